@@ -8,14 +8,34 @@
 // smaller), so the exact Cholesky factor L of A (L L^T = A, no pivoting, A
 // SPD) fits a band of b+1 diagonals and costs n b^2 / 2 multiply-adds:
 //
-//   band storage, column-major by diagonal: B[j (b+1) + d] = L(j+d, j),
-//   one block per wavenumber factors column by column (right-looking):
-//     L(j,j) = sqrt(a_jj);  L(j+i,j) = a_{j+i,j} / L(j,j);
-//     a_{j+i, j+l} -= L(j+i,j) L(j+l,j)   (1 <= l <= i <= b),
-//   then L y = b, L^T x = y for every column of the wavenumber (one thread
-//   per right-hand side, sequential over the band; for bandwidths up to 64
-//   the last b solution values stay in registers).  Bandwidths up to 31 are
-//   factored by one warp per wavenumber (lane d holds L(j+d, j)).
+// Blocks of B = max(b, 8) consecutive rows in band order make the matrix block
+// tridiagonal (N = ceil(n / B) dense blocks).  A serial band Cholesky has n
+// dependent columns and one substitution chain per right-hand side; block
+// cyclic reduction has log2(N) levels whose blocks are independent:
+//   level s (stride): every odd multiple i of s is eliminated between its
+//   neighbours l = i - s and r = i + s,
+//     V_l = D_i^-1 A(i,l),  V_r = D_i^-1 A(i,r),
+//     D_l -= A(l,i) V_l,  D_r -= A(r,i) V_r,  A(l,r) = -A(l,i) V_r,
+//     f_l -= V_l^T f_i,  f_r -= V_r^T f_i,
+//   then from the last level back x_i = D_i^-1 f_i - V_l x_l - V_r x_r.
+// Every D_i is a Schur complement of an SPD matrix (a symmetric permutation of
+// the Cholesky elimination), so its inverse by Gauss-Jordan needs no pivoting.
+//
+// Bound: the FP64 pipe (GB300: 1.2 TFLOP/s).  Per right-hand side the products
+// cost 10 n B flops against the 4 n b of the serial substitutions, and the
+// factor 11 n B^2 against n b^2, but every SM works on them.  Factor and solve,
+// serial -> reduction: 16 electrodes (n 684, 14 wavenumbers) 3.54 -> 0.26 ms; 41
+// electrodes (n 3618, b 19, 17 wavenumbers, 697 right-hand sides) 26.2 -> 1.15
+// ms; 72 electrodes on a fine mesh (n 25992, b 25, 1296 right-hand sides) 229.6
+// -> 11.7 ms, its widest level (k_cr_back, 2.2 ms) at 95 % of the FP64 rate.
+// The last levels hold few blocks; there the columns are split finer and the
+// inverse's chain of B dependent steps (25-38 us per level) is what remains.
+//
+// Blocks wider than kCrMax rows (their inverse and one operand would not fit
+// shared memory), and matrices whose 4 n B values per wavenumber do not fit the
+// device, take the serial band Cholesky: B[j (b+1) + d] = L(j+d, j), one
+// block per wavenumber factoring column by column, one thread per
+// right-hand side in the substitutions.
 //
 // Rows are visited in the chosen order through a permutation, so the
 // right-hand-side and solution blocks stay in the mesh's node order.  A pivot
@@ -85,90 +105,367 @@ __global__ void __launch_bounds__(kBandThreads) k_band_factor(int64_t n, int b, 
     }
 }
 
-// Narrow bands (b <= 31): one warp per wavenumber factors column by column
-// with lane d holding L(j+d, j); the update of the next columns is lane-
-// parallel, and __syncwarp orders it before the next column is read.
-__global__ void __launch_bounds__(128) k_band_factor_warp(int64_t n, int b, int nK, double *__restrict__ B,
-                                                           int32_t *__restrict__ bad) {
-    const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (w >= nK) return;
-    double *A = B + (int64_t)w * n * (b + 1);
-    for (int64_t j = 0; j < n; j++) {
-        const int m = (int)(n - 1 - j < (int64_t)b ? n - 1 - j : (int64_t)b);
-        double *Aj = A + j * (b + 1);
-        double v = lane <= m ? Aj[lane] : 0.0;
-        double d = __shfl_sync(0xffffffffu, v, 0);
-        if (!(d > 0.0) || !isfinite(d)) {
-            if (lane == 0) atomicAdd(bad, 1);
-            d = 1.0;
+// ------------------------------------------------ block cyclic reduction
+constexpr int kCrMax = 112;      // widest block: D and one operand in shared memory (2 x 100 KB)
+constexpr int kCrThreads = 256;
+constexpr int kCrChunk = 32;     // inner-dimension chunk of the right-hand-side products
+constexpr int kCrOut = 16;       // outputs per thread of the right-hand-side products, at most
+
+// Matrix blocks of every wavenumber: D (diagonal, later its inverse), C
+// (coupling of a block to the next active one), V_l and V_r, each N x B x B
+// row-major.
+struct CrMat {
+    double *D, *C, *VL, *VR;
+    int N, B;
+    __device__ double *d(int k, int i) const { return D + ((int64_t)k * N + i) * B * B; }
+    __device__ double *c(int k, int i) const { return C + ((int64_t)k * N + i) * B * B; }
+    __device__ double *vl(int k, int i) const { return VL + ((int64_t)k * N + i) * B * B; }
+    __device__ double *vr(int k, int i) const { return VR + ((int64_t)k * N + i) * B * B; }
+};
+
+__global__ void __launch_bounds__(kBandThreads) k_cr_fill(int64_t n, int nK, int64_t nnz,
+                                                           const int32_t *__restrict__ rowptr,
+                                                           const int32_t *__restrict__ colidx,
+                                                           const int32_t *__restrict__ pos,
+                                                           const double *__restrict__ S, CrMat m) {
+    const int64_t rows = (int64_t)m.N * m.B, total = rows * nK;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const int k = (int)(t / rows);
+        const int64_t i = t - k * rows;
+        if (i >= n) {  // rows past the matrix: identity
+            const int bi = (int)(i / m.B), r = (int)(i - (int64_t)bi * m.B);
+            m.d(k, bi)[r * m.B + r] = 1.0;
+            continue;
         }
-        const double ljj = sqrt(d);
-        v = lane == 0 ? ljj : v / ljj;
-        if (lane <= m) Aj[lane] = v;
-        for (int l = 1; l <= m; l++) {
-            const double cl = __shfl_sync(0xffffffffu, v, l);
-            if (lane >= l && lane <= m) A[(j + l) * (b + 1) + (lane - l)] -= v * cl;
+        const int pi = pos[i], bi = pi / m.B, r = pi - bi * m.B;
+        for (int32_t s = rowptr[i]; s < rowptr[i + 1]; s++) {
+            const int pj = pos[colidx[s]], bj = pj / m.B, c = pj - bj * m.B;
+            if (bj == bi) m.d(k, bi)[r * m.B + c] = S[(int64_t)k * nnz + s];
+            else if (bj == bi + 1) m.c(k, bi)[r * m.B + c] = S[(int64_t)k * nnz + s];
         }
-        __syncwarp();
     }
 }
 
-// Narrow bands (b <= BW): one thread per right-hand side, the last BW
-// solution values of its column in registers (pull form): forward
-// y_j = (r_j - sum_{i=1..b} L(j, j-i) y_{j-i}) / L_jj with L(j, j-i) =
-// B[(j-i)(b+1) + i], backward x_j = (y_j - sum_i L(j+i, j) x_{j+i}) / L_jj.
-template <int BW>
-__global__ void __launch_bounds__(128) k_band_solve_reg(int64_t n, int b, int nE, int64_t Rpad,
-                                                         const double *__restrict__ B,
-                                                         const int32_t *__restrict__ perm,
-                                                         double *__restrict__ x) {
-    const int k = blockIdx.y;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nE) return;
-    const double *L = B + (int64_t)k * n * (b + 1);
-    double *xc = x + (int64_t)k * nE + e;
-    double win[BW];
-#pragma unroll
-    for (int i = 0; i < BW; i++) win[i] = 0.0;  // win[i] = y_{j-1-i}
-    for (int64_t j = 0; j < n; j++) {
-        const int64_t row = perm[j];
-        double s0 = xc[row * Rpad], s1 = 0.0;
-#pragma unroll
-        for (int i = 0; i < BW; i++) {
-            const int64_t c = j - 1 - i;  // column j-1-i holds L(j, c) at offset i+1
-            if (i < b && c >= 0) {
-                const double l = L[c * (b + 1) + i + 1];
-                if (i & 1) s1 = fma(-l, win[i], s1);
-                else s0 = fma(-l, win[i], s0);
+// Elimination of block i = s + 2 s blockIdx.x: its inverse by Gauss-Jordan in
+// shared memory, then V_l and V_r.  A thread owns one column of the inverse and
+// every G-th row, so a step costs it one product and its rows' multiply-adds;
+// the pivot's reciprocal is taken once, by the thread that updated the pivot,
+// before the barrier that ends a step.  s = 0: the last block, inverse only.
+__global__ void __launch_bounds__(kCrThreads) k_cr_eliminate(CrMat m, int s, int32_t *__restrict__ bad) {
+    extern __shared__ double cr_smem[];
+    const int B = m.B, k = blockIdx.y, tid = threadIdx.x;
+    const int i = s ? s + 2 * s * (int)blockIdx.x : 0;
+    double *A = cr_smem, *X = A + B * B, *prow = X + B * (B + 1), *pcol = prow + 2 * B, *rd = pcol + 2 * B;
+    double *Di = m.d(k, i);
+    for (int q = tid; q < B * B; q += kCrThreads) A[q] = Di[q];
+    __syncthreads();
+    const int G = kCrThreads / B, g = tid / B, j = tid - g * B;  // B <= kCrThreads: G >= 1
+    auto reciprocal = [&](double d) {
+        if (!(d > 0.0) || !isfinite(d)) {
+            atomicAdd(bad, 1);
+            d = 1.0;
+        }
+        return 1.0 / d;
+    };
+    if (tid < B) {
+        prow[tid] = A[tid];
+        pcol[tid] = A[tid * B];
+        if (tid == 0) rd[0] = reciprocal(A[0]);
+    }
+    __syncthreads();
+    for (int p = 0; p < B; p++) {
+        const double *pr = prow + (p & 1) * B, *pc = pcol + (p & 1) * B;
+        double *nr = prow + ((p + 1) & 1) * B, *nc = pcol + ((p + 1) & 1) * B;
+        const double d = rd[p & 1];
+        if (g < G) {
+            const double f = pr[j] * d;  // the scaled pivot row at this thread's column
+            for (int r = g; r < B; r += G) {
+                double v;
+                if (r == p) v = j == p ? d : f;
+                else if (j == p) v = -pc[r] * d;
+                else v = fma(-pc[r], f, A[r * B + j]);
+                A[r * B + j] = v;
+                if (r == p + 1) {
+                    nr[j] = v;
+                    if (j == p + 1) rd[(p + 1) & 1] = reciprocal(v);
+                }
+                if (j == p + 1) nc[r] = v;
             }
         }
-        const double y = (s0 + s1) / L[j * (b + 1)];
-        xc[row * Rpad] = y;
-#pragma unroll
-        for (int i = BW - 1; i > 0; i--) win[i] = win[i - 1];
-        win[0] = y;
+        __syncthreads();
     }
-#pragma unroll
-    for (int i = 0; i < BW; i++) win[i] = 0.0;  // win[i] = x_{j+1+i}
-    for (int64_t j = n - 1; j >= 0; j--) {
-        const int64_t row = perm[j];
-        const double *Lj = L + j * (b + 1);
-        double s0 = xc[row * Rpad], s1 = 0.0;
-#pragma unroll
-        for (int i = 0; i < BW; i++) {
-            if (i < b && j + 1 + i < n) {
-                const double l = Lj[i + 1];
-                if (i & 1) s1 = fma(-l, win[i], s1);
-                else s0 = fma(-l, win[i], s0);
+    for (int q = tid; q < B * B; q += kCrThreads) Di[q] = A[q];
+    if (!s) return;
+    // V_l = D^-1 A(i,l) = D^-1 C[l]^T, V_r = D^-1 C[i]
+    const double *Cl = m.c(k, i - s), *Ci = m.c(k, i);
+    const int LD = B + 1;
+    for (int q = tid; q < B * B; q += kCrThreads) {
+        const int r = q / B;
+        X[(q - r * B) * LD + r] = Cl[q];
+    }
+    __syncthreads();
+    double *VL = m.vl(k, i), *VR = m.vr(k, i);
+    const bool right = i + s < m.N;
+    for (int pass = 0; pass < 2; pass++) {
+        double *V = pass ? VR : VL;
+        for (int q = tid; q < B * B; q += kCrThreads) {
+            const int r = q / B, c = q - r * B;
+            const double *a = A + r * B, *x = X + c;
+            double s0 = 0.0, s1 = 0.0;
+            int e = 0;
+            for (; e + 1 < B; e += 2) {
+                s0 = fma(a[e], x[e * LD], s0);
+                s1 = fma(a[e + 1], x[(e + 1) * LD], s1);
+            }
+            if (e < B) s0 = fma(a[e], x[e * LD], s0);
+            V[q] = s0 + s1;
+        }
+        if (pass || !right) break;
+        __syncthreads();
+        for (int q = tid; q < B * B; q += kCrThreads) {
+            const int r = q / B;
+            X[r * LD + (q - r * B)] = Ci[q];
+        }
+        __syncthreads();
+    }
+}
+
+// Tile of right-hand sides: columns [c0, c0 + nc) of wavenumber k.
+struct CrRhs {
+    const int32_t *perm;
+    double *x;
+    int64_t n, Rpad;
+    int nE, ntile;  // tiles per wavenumber
+};
+
+// acc += M F for one block product: M is B x B with element (row, q) at
+// M[q * B + row] (trans) or M[row * B + q]; F the nc columns of block fb.
+// Outputs o of a thread: (row, column) = divmod(tid + o kCrThreads, nc).
+template <int NO, bool TRANS>
+__device__ __forceinline__ void cr_product(const CrMat &m, const CrRhs &R, const double *__restrict__ M, int k, int fb,
+                                           int c0, int nc, double sign, double *Ms, double *Fs, const int (&ro)[NO],
+                                           const int (&co)[NO], double (&acc)[NO]) {
+    const int B = m.B, tid = threadIdx.x;
+    for (int q0 = 0; q0 < B; q0 += kCrChunk) {
+        const int qn = min(kCrChunk, B - q0);
+        __syncthreads();  // the previous chunk is consumed
+        for (int t = tid; t < qn * B; t += kCrThreads) {
+            if (TRANS) {
+                Ms[t] = sign * M[q0 * B + t];
+            } else {
+                const int r = t / qn, q = t - r * qn;
+                Ms[q * B + r] = sign * M[r * B + q0 + q];
             }
         }
-        const double xv = (s0 + s1) / Lj[0];
-        xc[row * Rpad] = xv;
+        for (int t = tid; t < qn * nc; t += kCrThreads) {
+            const int q = t / nc, c = t - q * nc;
+            const int64_t row = (int64_t)fb * B + q0 + q;
+            Fs[t] = row < R.n ? R.x[(int64_t)R.perm[row] * R.Rpad + (int64_t)k * R.nE + c0 + c] : 0.0;
+        }
+        __syncthreads();
+        for (int q = 0; q < qn; q++) {
 #pragma unroll
-        for (int i = BW - 1; i > 0; i--) win[i] = win[i - 1];
-        win[0] = xv;
+            for (int o = 0; o < NO; o++)
+                if (tid + o * kCrThreads < B * nc) acc[o] = fma(Ms[q * B + ro[o]], Fs[q * nc + co[o]], acc[o]);
+        }
     }
+}
+
+// Update of the kept block j = 2 s e by its eliminated neighbours: the matrix
+// part (blocks [0, n_kept)) and the right-hand-side part (the others, one tile
+// of columns each) of one level share a launch: neither reads what the other
+// writes.
+template <int NO>
+__global__ void __launch_bounds__(kCrThreads) k_cr_update(CrMat m, int s, int n_kept, CrRhs R) {
+    extern __shared__ double cr_smem[];
+    const int B = m.B, k = blockIdx.y, tid = threadIdx.x;
+    if ((int)blockIdx.x < n_kept) {
+        const int j = 2 * s * (int)blockIdx.x, i1 = j - s, i2 = j + s;
+        double *A = cr_smem, *X = A + B * B;
+        double *Dj = m.d(k, j), *Cj = m.c(k, j);
+        const int half = B * (B + 1) / 2;
+        // D_j -= P^T-or-P times V, symmetric: the lower triangle, mirrored
+        auto rank_update = [&](bool trans) {
+            for (int q = tid; q < half; q += kCrThreads) {
+                int r = (int)((sqrtf(8.0f * (float)q + 1.0f) - 1.0f) * 0.5f);
+                while ((r + 1) * (r + 2) / 2 <= q) r++;
+                while (r * (r + 1) / 2 > q) r--;
+                const int c = q - r * (r + 1) / 2;
+                const double *a = trans ? A + r : A + r * B;
+                const int st = trans ? B : 1;
+                double s0 = 0.0, s1 = 0.0;
+                int e = 0;
+                for (; e + 1 < B; e += 2) {
+                    s0 = fma(a[e * st], X[e * B + c], s0);
+                    s1 = fma(a[(e + 1) * st], X[(e + 1) * B + c], s1);
+                }
+                if (e < B) s0 = fma(a[e * st], X[e * B + c], s0);
+                const double v = Dj[r * B + c] - (s0 + s1);
+                Dj[r * B + c] = v;
+                Dj[c * B + r] = v;
+            }
+        };
+        if (i2 < m.N) {
+            const double *VL = m.vl(k, i2), *VR = m.vr(k, i2);
+            for (int q = tid; q < B * B; q += kCrThreads) {
+                A[q] = Cj[q];
+                X[q] = VL[q];
+            }
+            __syncthreads();
+            rank_update(false);
+            if (i2 + s < m.N) {
+                __syncthreads();
+                for (int q = tid; q < B * B; q += kCrThreads) X[q] = VR[q];
+                __syncthreads();
+                for (int q = tid; q < B * B; q += kCrThreads) {
+                    const int r = q / B, c = q - r * B;
+                    double s0 = 0.0, s1 = 0.0;
+                    int e = 0;
+                    for (; e + 1 < B; e += 2) {
+                        s0 = fma(A[r * B + e], X[e * B + c], s0);
+                        s1 = fma(A[r * B + e + 1], X[(e + 1) * B + c], s1);
+                    }
+                    if (e < B) s0 = fma(A[r * B + e], X[e * B + c], s0);
+                    Cj[q] = -(s0 + s1);
+                }
+            }
+        }
+        if (i1 >= 0) {
+            const double *C1 = m.c(k, i1), *VR = m.vr(k, i1);
+            __syncthreads();
+            for (int q = tid; q < B * B; q += kCrThreads) {
+                A[q] = C1[q];
+                X[q] = VR[q];
+            }
+            __syncthreads();
+            rank_update(true);
+        }
+        return;
+    }
+    // f_j -= V_r(i1)^T f_i1 + V_l(i2)^T f_i2
+    const int t = (int)blockIdx.x - n_kept, j = 2 * s * (t / R.ntile), i1 = j - s, i2 = j + s, tile = t % R.ntile;
+    const int c0 = (int)((int64_t)R.nE * tile / R.ntile), nc = (int)((int64_t)R.nE * (tile + 1) / R.ntile) - c0;
+    double *Ms = cr_smem, *Fs = Ms + kCrChunk * B;
+    int ro[NO], co[NO];
+    double acc[NO];
+#pragma unroll
+    for (int o = 0; o < NO; o++) {
+        const int q = tid + o * kCrThreads;
+        ro[o] = q / nc;
+        co[o] = q - ro[o] * nc;
+        acc[o] = 0.0;
+    }
+    if (i1 >= 0) cr_product<NO, true>(m, R, m.vr(k, i1), k, i1, c0, nc, -1.0, Ms, Fs, ro, co, acc);
+    if (i2 < m.N) cr_product<NO, true>(m, R, m.vl(k, i2), k, i2, c0, nc, -1.0, Ms, Fs, ro, co, acc);
+#pragma unroll
+    for (int o = 0; o < NO; o++) {
+        const int64_t row = (int64_t)j * B + ro[o];
+        if (tid + o * kCrThreads < B * nc && row < R.n)
+            R.x[(int64_t)R.perm[row] * R.Rpad + (int64_t)k * R.nE + c0 + co[o]] += acc[o];
+    }
+}
+
+// x_i = D_i^-1 f_i - V_l x_l - V_r x_r of the blocks eliminated at stride s
+// (s = 0: the last block, no neighbours); one tile of columns per block
+template <int NO>
+__global__ void __launch_bounds__(kCrThreads) k_cr_back(CrMat m, int s, CrRhs R) {
+    extern __shared__ double cr_smem[];
+    const int B = m.B, k = blockIdx.y, tid = threadIdx.x, tile = (int)blockIdx.x % R.ntile;
+    const int i = s ? s + 2 * s * ((int)blockIdx.x / R.ntile) : 0;
+    const int c0 = (int)((int64_t)R.nE * tile / R.ntile), nc = (int)((int64_t)R.nE * (tile + 1) / R.ntile) - c0;
+    double *Ms = cr_smem, *Fs = Ms + kCrChunk * B;
+    int ro[NO], co[NO];
+    double acc[NO];
+#pragma unroll
+    for (int o = 0; o < NO; o++) {
+        const int q = tid + o * kCrThreads;
+        ro[o] = q / nc;
+        co[o] = q - ro[o] * nc;
+        acc[o] = 0.0;
+    }
+    cr_product<NO, false>(m, R, m.d(k, i), k, i, c0, nc, 1.0, Ms, Fs, ro, co, acc);
+    if (s) {
+        cr_product<NO, false>(m, R, m.vl(k, i), k, i - s, c0, nc, -1.0, Ms, Fs, ro, co, acc);
+        if (i + s < m.N) cr_product<NO, false>(m, R, m.vr(k, i), k, i + s, c0, nc, -1.0, Ms, Fs, ro, co, acc);
+    }
+#pragma unroll
+    for (int o = 0; o < NO; o++) {
+        const int64_t row = (int64_t)i * B + ro[o];
+        if (tid + o * kCrThreads < B * nc && row < R.n)
+            R.x[(int64_t)R.perm[row] * R.Rpad + (int64_t)k * R.nE + c0 + co[o]] = acc[o];
+    }
+}
+
+// Column tiles of a level with nblk independent blocks per wavenumber: at most
+// kCrOut outputs per thread and 48 columns, narrower (8 at least) while the
+// launch has fewer than two blocks per SM.
+int cr_tiles(int B, int nE, int64_t blocks, int nsm) {
+    int nc = std::min(48, kCrOut * kCrThreads / B);
+    int nt = (nE + nc - 1) / nc;
+    while (blocks * nt < 2 * nsm && nE / (2 * nt) >= 8) nt *= 2;
+    return nt;
+}
+
+template <template <int> class F, typename... A> void by_outputs(int B, int nc, A &&...args) {
+    const int no = (B * nc + kCrThreads - 1) / kCrThreads;
+    if (no <= 2) F<2>::go(args...);
+    else if (no <= 4) F<4>::go(args...);
+    else if (no <= 8) F<8>::go(args...);
+    else F<kCrOut>::go(args...);
+}
+
+// The limit is per function, not per launch, and a batch solves its problems on
+// several host threads: always the same value, the widest block's need.
+template <class K> void allow_smem(K kern) {
+    constexpr int most = (int)sizeof(double) * (kCrMax * kCrMax + kCrMax * (kCrMax + 1) + 4 * kCrMax + 2);
+    ERTGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+}
+
+template <int NO> struct CrUpdateL {
+    static void go(dim3 g, size_t smem, cudaStream_t st, const CrMat &m, int s, int n_kept, const CrRhs &R) {
+        allow_smem(k_cr_update<NO>);
+        k_cr_update<NO><<<g, kCrThreads, smem, st>>>(m, s, n_kept, R);
+    }
+};
+template <int NO> struct CrBackL {
+    static void go(dim3 g, size_t smem, cudaStream_t st, const CrMat &m, int s, const CrRhs &R) {
+        allow_smem(k_cr_back<NO>);
+        k_cr_back<NO><<<g, kCrThreads, smem, st>>>(m, s, R);
+    }
+};
+
+// Factor and solve; x holds the right-hand sides and receives the solution.
+// Returns the kernels launched.
+int cr_solve(Context &c, CrMat m, const int32_t *perm, double *x, int32_t *bad, cudaStream_t st) {
+    const int B = m.B, N = m.N, nK = c.nK;
+    int nsm = 0, launches = 0;
+    ERTGB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
+    const size_t elim = sizeof(double) * ((size_t)B * B + (size_t)B * (B + 1) + 4 * B + 2);
+    allow_smem(k_cr_eliminate);
+    auto rhs_smem = [&](int nc) { return sizeof(double) * (size_t)kCrChunk * (B + nc); };
+    std::vector<int> strides;
+    for (int s = 1; s < N; s *= 2) strides.push_back(s);
+    CrRhs R{perm, x, c.mesh.n, c.Rpad, c.nE, 1};
+    for (int s : strides) {
+        const int n_elim = (N - 1 - s) / (2 * s) + 1, n_kept = (N - 1) / (2 * s) + 1;
+        k_cr_eliminate<<<dim3((unsigned)n_elim, (unsigned)nK), kCrThreads, elim, st>>>(m, s, bad);
+        R.ntile = cr_tiles(B, c.nE, (int64_t)n_kept * nK, nsm);
+        const int nc = (c.nE + R.ntile - 1) / R.ntile;
+        const size_t smem = std::max(sizeof(double) * 2 * (size_t)B * B, rhs_smem(nc));
+        by_outputs<CrUpdateL>(B, nc, dim3((unsigned)(n_kept * (1 + R.ntile)), (unsigned)nK), smem, st, m, s, n_kept, R);
+        launches += 2;
+    }
+    k_cr_eliminate<<<dim3(1, (unsigned)nK), kCrThreads, elim, st>>>(m, 0, bad);
+    auto back = [&](int s) {  // s = 0: the last block
+        const int nblk = s ? (N - 1 - s) / (2 * s) + 1 : 1;
+        R.ntile = cr_tiles(B, c.nE, (int64_t)nblk * nK, nsm);
+        const int nc = (c.nE + R.ntile - 1) / R.ntile;
+        by_outputs<CrBackL>(B, nc, dim3((unsigned)(nblk * R.ntile), (unsigned)nK), rhs_smem(nc), st, m, s, R);
+    };
+    back(0);
+    for (size_t l = strides.size(); l-- > 0;) back(strides[l]);
+    ERTGB_CUDA(cudaGetLastError());
+    return launches + 2 + (int)strides.size();
 }
 
 // one block per wavenumber, one thread per right-hand side of it: forward
@@ -283,33 +580,41 @@ int band_solve(Context &c, cudaStream_t s) {
                                          std::to_string(kMaxBand) + " (this matrix: " + std::to_string(P.b) +
                                          "); use an iterative preconditioner");
     const int64_t n = m.n, b = P.b;
-    const size_t per = (size_t)n * (size_t)(b + 1);
-    c.d_band.alloc(per * c.nK);
-    ERTGB_CUDA(cudaMemsetAsync(c.d_band.p, 0, sizeof(double) * per * c.nK, s));
-    k_band_fill<<<(unsigned)std::min<int64_t>(ceil_div(n * c.nK, kBandThreads), 4096), kBandThreads, 0, s>>>(n, (int)b, c.nK, m.nnz, m.d_rowptr.p, m.d_colidx.p,
-                                                              P.d_pos.p, c.d_S.p, c.d_band.p);
     DBuf<int32_t> &bad = c.d_ic_bad;
     bad.alloc(1);
     bad.zero(s);
-    if (b <= 31)
-        k_band_factor_warp<<<(unsigned)ceil_div((int64_t)c.nK * 32, 128), 128, 0, s>>>(n, (int)b, c.nK, c.d_band.p,
-                                                                                        bad.p);
-    else
-        k_band_factor<<<c.nK, kBandThreads, 0, s>>>(n, (int)b, c.d_band.p, bad.p);
     // the solution overwrites a copy of the right-hand sides (d_r keeps them)
     c.d_x.alloc((size_t)n * c.Rpad);
     ERTGB_CUDA(cudaMemcpyAsync(c.d_x.p, c.d_r.p, sizeof(double) * n * c.Rpad, cudaMemcpyDeviceToDevice, s));
-    const dim3 sg((unsigned)ceil_div(c.nE, 32), (unsigned)c.nK);
-    if (b <= 16)
-        k_band_solve_reg<16><<<sg, 32, 0, s>>>(n, (int)b, c.nE, c.Rpad, c.d_band.p, P.d_perm.p, c.d_x.p);
-    else if (b <= 32)
-        k_band_solve_reg<32><<<sg, 32, 0, s>>>(n, (int)b, c.nE, c.Rpad, c.d_band.p, P.d_perm.p, c.d_x.p);
-    else if (b <= 64)
-        k_band_solve_reg<64><<<sg, 32, 0, s>>>(n, (int)b, c.nE, c.Rpad, c.d_band.p, P.d_perm.p, c.d_x.p);
-    else
+    const int B = (int)std::max<int64_t>(b, 8), N = (int)ceil_div(n, B);
+    const size_t blk = (size_t)c.nK * N * B * B;
+    bool reduction = B <= kCrMax;
+    if (reduction) {
+        try {
+            c.d_band.alloc(4 * blk);
+        } catch (Error &e) {
+            if (e.code != ERTGB_OOM) throw;
+            cudaGetLastError();  // a failed allocation: the serial form needs a quarter of it
+            reduction = false;
+        }
+    }
+    if (reduction) {
+        const CrMat M{c.d_band.p, c.d_band.p + blk, c.d_band.p + 2 * blk, c.d_band.p + 3 * blk, N, B};
+        ERTGB_CUDA(cudaMemsetAsync(M.D, 0, sizeof(double) * 2 * blk, s));
+        k_cr_fill<<<(unsigned)std::min<int64_t>(ceil_div((int64_t)N * B * c.nK, kBandThreads), 4096), kBandThreads, 0,
+                    s>>>(n, c.nK, m.nnz, m.d_rowptr.p, m.d_colidx.p, P.d_pos.p, c.d_S.p, M);
+        c.stats.launches_response += 1 + cr_solve(c, M, P.d_perm.p, c.d_x.p, bad.p, s);
+    } else {
+        const size_t per = (size_t)n * (size_t)(b + 1);
+        c.d_band.alloc(per * c.nK);
+        ERTGB_CUDA(cudaMemsetAsync(c.d_band.p, 0, sizeof(double) * per * c.nK, s));
+        k_band_fill<<<(unsigned)std::min<int64_t>(ceil_div(n * c.nK, kBandThreads), 4096), kBandThreads, 0, s>>>(
+            n, (int)b, c.nK, m.nnz, m.d_rowptr.p, m.d_colidx.p, P.d_pos.p, c.d_S.p, c.d_band.p);
+        k_band_factor<<<c.nK, kBandThreads, 0, s>>>(n, (int)b, c.d_band.p, bad.p);
         k_band_solve<<<c.nK, std::min(kBandThreads, ((c.nE + 31) / 32) * 32), 0, s>>>(n, (int)b, c.nE, c.Rpad,
-                                                                                      c.d_band.p, P.d_perm.p,
-                                                                                      c.d_x.p);
+                                                                                      c.d_band.p, P.d_perm.p, c.d_x.p);
+        c.stats.launches_response += 3;
+    }
     ERTGB_CUDA(cudaGetLastError());
     int32_t h = 0;
     ERTGB_CUDA(cudaMemcpyAsync(&h, bad.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
@@ -317,7 +622,6 @@ int band_solve(Context &c, cudaStream_t s) {
     c.stats.iterations = 0;
     c.stats.max_rel_residual = 0.0;
     c.stats.n_rhs = (int32_t)c.R;
-    c.stats.launches_response += 3;
     if (h) throw Error(ERTGB_NOT_CONVERGED, "banded Cholesky: " + std::to_string(h) + " pivots not positive");
     return ERTGB_OK;
 }
