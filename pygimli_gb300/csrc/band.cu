@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kBandThreads) k_band_factor(int64_t n, int b, 
 }
 
 // ------------------------------------------------ block cyclic reduction
-constexpr int kCrMax = 112;      // widest block: D and one operand in shared memory (2 x 100 KB)
+constexpr int kCrMax = kDenseMax;  // widest block: D and one operand in shared memory (2 x 100 KB)
 constexpr int kCrThreads = 256;
 constexpr int kCrChunk = 32;     // inner-dimension chunk of the right-hand-side products
 constexpr int kCrOut = 16;       // outputs per thread of the right-hand-side products, at most
@@ -414,11 +414,15 @@ template <template <int> class F, typename... A> void by_outputs(int B, int nc, 
     else F<kCrOut>::go(args...);
 }
 
+// the inverse, one operand, two pivot rows and columns, two reciprocals
+size_t eliminate_smem(int B) {
+    return sizeof(double) * ((size_t)B * B + (size_t)B * (B + 1) + 4 * B + 2);
+}
+
 // The limit is per function, not per launch, and a batch solves its problems on
 // several host threads: always the same value, the widest block's need.
 template <class K> void allow_smem(K kern) {
-    constexpr int most = (int)sizeof(double) * (kCrMax * kCrMax + kCrMax * (kCrMax + 1) + 4 * kCrMax + 2);
-    ERTGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    ERTGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eliminate_smem(kCrMax)));
 }
 
 template <int NO> struct CrUpdateL {
@@ -440,7 +444,7 @@ int cr_solve(Context &c, CrMat m, const int32_t *perm, double *x, int32_t *bad, 
     const int B = m.B, N = m.N, nK = c.nK;
     int nsm = 0, launches = 0;
     ERTGB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
-    const size_t elim = sizeof(double) * ((size_t)B * B + (size_t)B * (B + 1) + 4 * B + 2);
+    const size_t elim = eliminate_smem(B);
     allow_smem(k_cr_eliminate);
     auto rhs_smem = [&](int nc) { return sizeof(double) * (size_t)kCrChunk * (B + nc); };
     std::vector<int> strides;
@@ -570,6 +574,13 @@ void band_plan(Context &c) {
 }
 
 }  // namespace
+
+void dense_inverse(double *A, int n, int32_t *bad, cudaStream_t s) {
+    const CrMat M{A, nullptr, nullptr, nullptr, 1, n};
+    allow_smem(k_cr_eliminate);
+    k_cr_eliminate<<<1, kCrThreads, eliminate_smem(n), s>>>(M, 0, bad);
+    ERTGB_CUDA(cudaGetLastError());
+}
 
 int band_solve(Context &c, cudaStream_t s) {
     MeshData &m = c.mesh;

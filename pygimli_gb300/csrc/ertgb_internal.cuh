@@ -83,6 +83,38 @@ struct BandPlan {
     DBuf<int32_t> d_perm, d_pos;
 };
 
+// One level of the multilevel preconditioner on the host (coarsen.cpp): its
+// matrix pattern, the prolongation P (n x nc) with its transpose, and the
+// pattern of A P.  The last level has a matrix pattern only.
+struct HostLevel {
+    int64_t n = 0, nc = 0;
+    std::vector<int32_t> rp, ci, P_rp, P_ci, PT_rp, PT_ci, AP_rp, AP_ci;
+    std::vector<float> P_v, PT_v;
+};
+
+// The same on the device (multilevel.cu) with the values of the current model
+// and the level's vectors.  Level 0 uses the mesh's pattern and matrix.
+struct MlLevel {
+    int64_t n = 0, nc = 0, nnz = 0, nnzP = 0, nnzAP = 0;
+    DBuf<int32_t> rp, ci, P_rp, P_ci, PT_rp, PT_ci, AP_rp, AP_ci;
+    DBuf<float> P_v, PT_v;
+    DBuf<double> val, AP;   // FP64 matrix (levels >= 1) and A P
+    DBuf<float> AS, Q, dw;  // A diag(dw); the post-smoothed prolongation (or -A P); the rows' damping
+    DBuf<float> b, r, e;    // right-hand side, residual, correction: n x Rpad
+};
+
+struct Multilevel {
+    bool tried = false, ok = false;  // built for this mesh / usable
+    std::vector<uint8_t> fixed;      // the fixed rows it was built with
+    std::vector<std::unique_ptr<MlLevel>> levels;  // the coarsest last
+    DBuf<double> inv64;              // coarsest inverse
+    DBuf<float> inv32;
+    DBuf<int32_t> bad;
+    bool factor = false;             // fine-level smoother: the factor G^T G (else Jacobi)
+    DBuf<float> w, px, pt, pg;       // the factor's damping; power iteration vectors (n x 32)
+    DBuf<double> ppart;
+};
+
 // Mesh-dependent structures.
 struct MeshData {
     int dim = 0, order = 1, nv = 0, nvb = 0;  // nv / nvb: nodes per cell / boundary
@@ -101,6 +133,7 @@ struct MeshData {
     DBuf<int32_t> d_Lrowptr, d_Lcolidx, d_LtoA, d_Urowptr, d_Ucolidx, d_UtoL;
     Ic0Plan ic0;  // built on first use of the IC(0) preconditioner
     BandPlan band;  // built on first use of the banded direct solve
+    Multilevel ml;  // built on first use of the mixed-precision solver on a 3-D mesh
     // device
     DBuf<double> d_xyz;
     DBuf<int32_t> d_cells, d_rowptr, d_colidx, d_diag;
@@ -278,6 +311,7 @@ struct Context {
     DBuf<double> d_S;             // nK x nnz
     DBuf<double> d_dinv;          // nK x n  (1 / diag)
     DBuf<double> d_pnorm2;        // Rpad: ||S1 u_p / rho_s||^2 per right-hand side (convergence reference floor)
+    bool pnorm_ready = false;     // d_pnorm2 belongs to the current S1 and primary potentials
     DBuf<double> d_rhos;          // nE source resistivity
     DBuf<double> d_x, d_r, d_p, d_q;  // n x Rpad (d_r holds the right-hand sides)
     // mixed precision: FP32 matrix, Jacobi diagonal and recurrence vectors
@@ -394,6 +428,20 @@ void build_assembly_map(MeshData &m, std::vector<int32_t> &cptr, std::vector<int
 void build_jacobian_tiles(Context &c);
 void build_lower_pattern(MeshData &m);
 void build_extension_map(const MeshData &m, std::vector<int32_t> &ptr, std::vector<double> &val);
+// coarsen.cpp: coarse levels from a unit-resistivity matrix, down to at most
+// ``coarsest`` rows; false: no useful hierarchy
+bool build_levels(const std::vector<int32_t> &rowptr, const std::vector<int32_t> &colidx,
+                  const std::vector<double> &unit, int64_t coarsest, int max_levels, std::vector<HostLevel> &out);
+// multilevel.cu: coarse levels of the current matrix (d_S; the preconditioner's
+// factor in d_G32 when ``factor``); false: the single-level preconditioner
+// stays.  ml_cycle: d_z32 = M^-1 d_r32 with the column partials of r . z (NB
+// block rows) in pz.
+bool ml_setup(Context &c, bool factor, cudaStream_t s);
+void ml_cycle(Context &c, int NB, double *pz, cudaStream_t s);
+int ml_launches(const Context &c);
+// band.cu: inverse of one SPD matrix of at most 112 rows, in place (one block)
+constexpr int kDenseMax = 112;
+void dense_inverse(double *A, int n, int32_t *bad, cudaStream_t s);
 // fsai.cu
 void fsai_setup(Context &c, cudaStream_t s);
 // ic0.cu: factor every wavenumber's matrix (d_S) into d_ic; z = (L L^T)^-1 r

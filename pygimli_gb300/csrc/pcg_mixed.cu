@@ -24,6 +24,7 @@ namespace {
 constexpr int kRows = 8;            // warps per block (spmm) / rows per block (vector kernels)
 constexpr int kGraphIters = 16;     // iterations per captured graph
 constexpr int kReliableEvery = 4;   // graphs between reliable updates (64 iterations)
+constexpr int kMlIters = 6;         // iterations per graph with coarse levels, the last a reliable update
 constexpr int kPartRows = 304;  // 2 row blocks per SM: few partial rows keep the column finishes short
 
 
@@ -365,14 +366,44 @@ __global__ void k_m_accum(int64_t n, int64_t Rpad, const int32_t *__restrict__ a
     }
 }
 
+// Coarse levels: the last iteration of a graph is the reliable update.  Its
+// first part, x += y + alpha p and y = 0
+__global__ void k_m_accum_p(int64_t n, int64_t Rpad, const double *__restrict__ col, const int32_t *__restrict__ active,
+                            double *__restrict__ x, float *__restrict__ y, const float *__restrict__ p) {
+    const int64_t t = (int64_t)blockIdx.x * 32 + threadIdx.x;
+    if (!active[t]) return;
+    const float alpha = (float)col[ALPHA * Rpad + t];
+#pragma unroll 4
+    for (int64_t row = (int64_t)blockIdx.y * kRows + threadIdx.y; row < n; row += (int64_t)gridDim.y * kRows) {
+        const int64_t i = row * Rpad + t;
+        x[i] += (double)y[i] + (double)alpha * (double)p[i];
+        y[i] = 0.f;
+    }
+}
+
+// its last part: p = z + beta p
+__global__ void k_m_update_pz(int64_t n, int64_t Rpad, const double *__restrict__ col, const int32_t *__restrict__ active,
+                              const float *__restrict__ z, float *__restrict__ p) {
+    const int64_t t = (int64_t)blockIdx.x * 32 + threadIdx.x;
+    if (!active[t]) return;
+    const float beta = (float)col[BETA * Rpad + t];
+#pragma unroll 4
+    for (int64_t row = (int64_t)blockIdx.y * kRows + threadIdx.y; row < n; row += (int64_t)gridDim.y * kRows) {
+        const int64_t i = row * Rpad + t;
+        p[i] = fmaf(beta, p[i], z[i]);
+    }
+}
+
 // reliable update, part 2: true residual r = b - A x in FP64 (warp per row,
-// lanes over columns), restart r32 from it, partials of r32.z32 and ||r||^2
+// lanes over columns), restart r32 from it, partials of r32.z32 and ||r||^2.
+// zold (coarse levels): the first partial is zold . r instead of r . D^-1 r
 template <int CH>
 __global__ void __launch_bounds__(256) k_m_residual(int64_t n, int64_t nnz, int nE, int nK, int64_t R, int64_t Rpad,
                                                     const int32_t *__restrict__ rowptr,
                                                     const int32_t *__restrict__ colidx,
                                                     const double *__restrict__ vals, const double *__restrict__ x,
                                                     const double *__restrict__ b, const float *__restrict__ dinv,
+                                                    const float *__restrict__ zold,
                                                     const int32_t *__restrict__ active, float *__restrict__ r32,
                                                     double *__restrict__ part_a, double *__restrict__ part_b) {
     __shared__ double ra[kRows][32 * CH], rb[kRows][32 * CH];
@@ -410,7 +441,7 @@ __global__ void __launch_bounds__(256) k_m_residual(int64_t n, int64_t nnz, int 
             const double rv = b[i] - acc[j];
             const float r = (float)rv;
             r32[i] = r;
-            sa[j] += (double)(r * (r * dinv[kdi[j] + row]));
+            sa[j] += zold ? (double)(zold[i] * r) : (double)(r * (r * dinv[kdi[j] + row]));
             sb[j] = fma(rv, rv, sb[j]);
         }
     }
@@ -450,6 +481,61 @@ __global__ void k_m_finish_ru(int64_t Rpad, int NB, double rtol2, const double *
     const double bb = col[BNORM2 * Rpad + t];
     col[RNORM2 * Rpad + t] = rr;
     col[RHO * Rpad + t] = rz;
+    if (rr <= rtol2 * bb) {
+        cs.active[t] = 0;
+        return;
+    }
+    if (!(rr <= 4.0 * bb) || !(rz == rz)) {  // diverged or not finite
+        cs.active[t] = 0;
+        cs.stalled[t] = 2;
+        atomicAdd(cs.nstalled, 1);
+        return;
+    }
+    const double best = col[RPREV * Rpad + t];
+    double stalls = col[STALLS * Rpad + t];
+    if (rr < 0.81 * best) {
+        col[RPREV * Rpad + t] = rr;
+        stalls = 0.0;
+    } else {
+        stalls += 1.0;
+    }
+    col[STALLS * Rpad + t] = stalls;
+    if (stalls >= 4.0) {
+        cs.active[t] = 0;
+        cs.stalled[t] = 1;
+        atomicAdd(cs.nstalled, 1);
+        return;
+    }
+    atomicAdd(cs.nactive, 1);
+}
+
+// Coarse levels: convergence test on the true residual and the next direction.
+// part_a: r . z, part_b: ||r||^2, part_c: zold . r, zero in exact CG.  A
+// multilevel interval can gain more digits than FP32 carries; the true residual
+// then differs from the recursive one and the old direction is no longer
+// conjugate to it.  beta is therefore (r . z - zold . r) / rho, or zero (a restart
+// from the true residual) where |zold . r| > 0.2 r . z (Powell, Math.
+// Programming 12, 1977).  Without it a fast problem diverged after 12 iterations
+// between updates.
+__global__ void k_m_finish_ml(int64_t Rpad, int NB, double rtol2, const double *__restrict__ part_a,
+                              const double *__restrict__ part_b, const double *__restrict__ part_c,
+                              double *__restrict__ col, ColState cs) {
+    const int64_t t = (int64_t)blockIdx.x * kFinWarps + (threadIdx.x >> 5);
+    if (t >= Rpad) return;
+    const double rz = warp_col_sum(part_a, NB, Rpad, t);
+    const double rr = warp_col_sum(part_b, NB, Rpad, t);
+    const double zr = warp_col_sum(part_c, NB, Rpad, t);
+    if ((threadIdx.x & 31) != 0) return;
+    if (!cs.active[t]) {
+        col[BETA * Rpad + t] = 0.0;
+        return;
+    }
+    cs.iters[t] += 1;
+    const double rho = col[RHO * Rpad + t], bb = col[BNORM2 * Rpad + t];
+    const bool keep = rho > 0.0 && rz > 0.0 && fabs(zr) <= 0.2 * rz;
+    col[BETA * Rpad + t] = keep ? (rz - zr) / rho : 0.0;
+    col[RHO * Rpad + t] = rz;
+    col[RNORM2 * Rpad + t] = rr;
     if (rr <= rtol2 * bb) {
         cs.active[t] = 0;
         return;
@@ -530,8 +616,8 @@ template <int CH> struct GenL {
 template <int CH> struct ResidL {
     static void go(dim3 g, cudaStream_t s, int64_t n, int64_t nnz, int nE, int nK, int64_t R, int64_t Rpad,
                    const int32_t *rp, const int32_t *ci, const double *v, const double *x, const double *b,
-                   const float *dinv, const int32_t *active, float *r32, double *pa, double *pb) {
-        k_m_residual<CH><<<g, 256, 0, s>>>(n, nnz, nE, nK, R, Rpad, rp, ci, v, x, b, dinv, active, r32, pa, pb);
+                   const float *dinv, const float *zold, const int32_t *active, float *r32, double *pa, double *pb) {
+        k_m_residual<CH><<<g, 256, 0, s>>>(n, nnz, nE, nK, R, Rpad, rp, ci, v, x, b, dinv, zold, active, r32, pa, pb);
     }
 };
 
@@ -567,8 +653,17 @@ int pcg_solve_mixed(Context &c, cudaStream_t s) {
         c.d_t32.alloc((size_t)n * Rpad);
         c.d_z32.alloc((size_t)n * Rpad);
     }
-    // z = G^T (G r) with the column partials of r . z into pz
+    k_to_f32<<<(unsigned)std::min<int64_t>(ceil_div((int64_t)c.nK * m.nnz, 256), 65535), 256, 0, s>>>(
+        (int64_t)c.nK * m.nnz, c.d_S.p, c.d_S32.p);
+    const bool ml = ml_setup(c, fsai, s);  // coarse levels around the factor (or Jacobi)
+    const bool zform = fsai || ml;         // z = M^-1 r is a product of its own
+    // z = M^-1 r with the column partials of r . z into pz: the multilevel
+    // cycle, or G^T (G r)
     auto apply_fsai = [&](double *pz) {
+        if (ml) {
+            ml_cycle(c, NB, pz, s);
+            return;
+        }
         dispatch_ch<GenL>(ch, dim3((unsigned)NB, (unsigned)nchunk), s, n, nL, c.nE, c.nK, Rpad, m.d_Lrowptr.p,
                           m.d_Lcolidx.p, c.d_G32.p, c.d_r32.p, c.d_t32.p, (const float *)nullptr, (double *)nullptr);
         dispatch_ch<GenL>(ch, dim3((unsigned)NB, (unsigned)nchunk), s, n, nL, c.nE, c.nK, Rpad, m.d_Urowptr.p,
@@ -576,8 +671,6 @@ int pcg_solve_mixed(Context &c, cudaStream_t s) {
     };
     ERTGB_CUDA(cudaMemsetAsync(c.d_x.p, 0, sizeof(double) * n * Rpad, s));
     ERTGB_CUDA(cudaMemsetAsync(cs.stalled, 0, sizeof(int32_t) * (Rpad + 2), s));  // stalled flags + counters
-    k_to_f32<<<(unsigned)std::min<int64_t>(ceil_div((int64_t)c.nK * m.nnz, 256), 65535), 256, 0, s>>>(
-        (int64_t)c.nK * m.nnz, c.d_S.p, c.d_S32.p);
     k_to_f32<<<(unsigned)std::min<int64_t>(ceil_div((int64_t)c.nK * n, 256), 65535), 256, 0, s>>>(
         (int64_t)c.nK * n, c.d_dinv.p, c.d_dinv32.p);
     const dim3 vb(32, kRows), vg((unsigned)(Rpad / 32), (unsigned)NB);
@@ -588,10 +681,10 @@ int pcg_solve_mixed(Context &c, cudaStream_t s) {
     const unsigned fwg = (unsigned)ceil_div(Rpad, kFinWarps);
     const double rtol2 = c.rtol * c.rtol;
     k_m_init<<<vg, vb, 0, s>>>(n, c.nE, R, Rpad, c.d_dinv32.p, b, c.d_r32.p, c.d_p32.p, c.d_y32.p, part_a, part_b);
-    if (fsai) {
+    if (zform) {
         apply_fsai(part_a);
         ERTGB_CUDA(cudaMemcpyAsync(c.d_p32.p, c.d_z32.p, sizeof(float) * n * Rpad, cudaMemcpyDeviceToDevice, s));
-        c.stats.launches_response += 2;
+        c.stats.launches_response += ml ? ml_launches(c) : 2;
     }
     pcg_finish_init(fg, fb, s, Rpad, R, NB, part_a, part_b, c.d_col.p, active, iters, nactive,
                     c.d_pnorm2.n >= (size_t)Rpad ? c.d_pnorm2.p : nullptr);
@@ -613,6 +706,9 @@ int pcg_solve_mixed(Context &c, cudaStream_t s) {
         }
     }
 
+    // a multilevel iteration gains about a third of a digit: a reliable update
+    // (and convergence test) every 6, against every 64 without coarse levels
+    const int graph_iters = ml ? kMlIters : kGraphIters, reliable = ml ? 1 : kReliableEvery;
     cudaGraph_t g_it = nullptr, g_ru = nullptr;
     cudaGraphExec_t e_it = nullptr, e_ru = nullptr;
     auto cleanup = [&] {
@@ -625,11 +721,18 @@ int pcg_solve_mixed(Context &c, cudaStream_t s) {
     int iterations = 0;
     try {
         ERTGB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        for (int it = 0; it < kGraphIters; it++) {
+        for (int it = 0; it < graph_iters; it++) {
             dispatch_ch<SpmmL>(ch, sg, s, n, m.nnz, c.nE, c.nK, Rpad, m.d_rowptr.p, m.d_colidx.p, c.d_S32.p, c.d_p32.p,
                                c.d_q32.p, part_c);
             k_m_finish_alpha_w<<<fwg, 32 * kFinWarps, 0, s>>>(Rpad, NB, part_c, c.d_col.p, active, nactive);
-            if (fsai) {
+            if (ml && it + 1 == graph_iters) {
+                k_m_accum_p<<<vgu, vb, 0, s>>>(n, Rpad, c.d_col.p, active, c.d_x.p, c.d_y32.p, c.d_p32.p);
+                dispatch_ch<ResidL>(ch, sg, s, n, m.nnz, c.nE, c.nK, R, Rpad, m.d_rowptr.p, m.d_colidx.p, c.d_S.p,
+                                    c.d_x.p, b, c.d_dinv32.p, c.d_z32.p, active, c.d_r32.p, part_c, part_b);
+                apply_fsai(part_a);
+                k_m_finish_ml<<<fwg, 32 * kFinWarps, 0, s>>>(Rpad, NB, rtol2, part_a, part_b, part_c, c.d_col.p, cs);
+                k_m_update_pz<<<vgu, vb, 0, s>>>(n, Rpad, c.d_col.p, active, c.d_z32.p, c.d_p32.p);
+            } else if (zform) {
                 k_m_update_r<<<vgu, vb, 0, s>>>(n, Rpad, c.d_col.p, active, c.d_r32.p, c.d_q32.p);
                 apply_fsai(part_a);
                 k_m_finish_beta_w<<<fwg, 32 * kFinWarps, 0, s>>>(Rpad, NB, part_a, c.d_col.p, active, iters);
@@ -644,14 +747,16 @@ int pcg_solve_mixed(Context &c, cudaStream_t s) {
         }
         ERTGB_CUDA(cudaStreamEndCapture(s, &g_it));
         ERTGB_CUDA(cudaGraphInstantiate(&e_it, g_it, 0));
-        ERTGB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        k_m_accum<<<vg, vb, 0, s>>>(n, Rpad, active, c.d_x.p, c.d_y32.p, nactive);
-        dispatch_ch<ResidL>(ch, sg, s, n, m.nnz, c.nE, c.nK, R, Rpad, m.d_rowptr.p, m.d_colidx.p, c.d_S.p, c.d_x.p,
-                            b, c.d_dinv32.p, active, c.d_r32.p, part_a, part_b);
-        if (fsai) apply_fsai(part_a);
-        k_m_finish_ru<<<fg, fb, 0, s>>>(Rpad, NB, rtol2, part_a, part_b, c.d_col.p, cs);
-        ERTGB_CUDA(cudaStreamEndCapture(s, &g_ru));
-        ERTGB_CUDA(cudaGraphInstantiate(&e_ru, g_ru, 0));
+        if (!ml) {
+            ERTGB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+            k_m_accum<<<vg, vb, 0, s>>>(n, Rpad, active, c.d_x.p, c.d_y32.p, nactive);
+            dispatch_ch<ResidL>(ch, sg, s, n, m.nnz, c.nE, c.nK, R, Rpad, m.d_rowptr.p, m.d_colidx.p, c.d_S.p, c.d_x.p,
+                                b, c.d_dinv32.p, nullptr, active, c.d_r32.p, part_a, part_b);
+            if (fsai) apply_fsai(part_a);
+            k_m_finish_ru<<<fg, fb, 0, s>>>(Rpad, NB, rtol2, part_a, part_b, c.d_col.p, cs);
+            ERTGB_CUDA(cudaStreamEndCapture(s, &g_ru));
+            ERTGB_CUDA(cudaGraphInstantiate(&e_ru, g_ru, 0));
+        }
 
         int32_t h_active = 0;
         ERTGB_CUDA(cudaMemcpyAsync(&h_active, nactive, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
@@ -661,10 +766,14 @@ int pcg_solve_mixed(Context &c, cudaStream_t s) {
                 status = ERTGB_NOT_CONVERGED;
                 break;
             }
-            for (int u = 0; u < kReliableEvery; u++) ERTGB_CUDA(cudaGraphLaunch(e_it, s));
-            iterations += kReliableEvery * kGraphIters;
-            ERTGB_CUDA(cudaGraphLaunch(e_ru, s));
-            c.stats.launches_response += (fsai ? 6 : 5) * kGraphIters * kReliableEvery + (fsai ? 5 : 3);
+            for (int u = 0; u < reliable; u++) ERTGB_CUDA(cudaGraphLaunch(e_it, s));
+            iterations += reliable * graph_iters;
+            if (ml) {
+                c.stats.launches_response += (5 + ml_launches(c)) * graph_iters + 1;
+            } else {
+                ERTGB_CUDA(cudaGraphLaunch(e_ru, s));
+                c.stats.launches_response += (fsai ? 6 : 5) * graph_iters * reliable + (fsai ? 5 : 3);
+            }
             ERTGB_CUDA(cudaMemcpyAsync(&h_active, nactive, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
             ERTGB_CUDA(cudaStreamSynchronize(s));
         }

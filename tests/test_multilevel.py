@@ -1,0 +1,138 @@
+"""Coarse levels of the mixed-precision solver (3-D meshes of at least 1024
+nodes) against the plain FP64 PCG at rtol 1e-12: every fine-level smoother,
+ground and boundary condition that the solver takes, repeated passes on one
+operator, changed models and fixed rows.
+
+Tolerance: both runs stop on the same true residual test, the mixed one at
+rtol 1e-10; the repository's accuracy table puts the potentials within 1e-10 of
+the column maximum there, and the bar is 100 times that."""
+import os
+
+import numpy as np
+import pytest
+
+from pygimli_gb300 import DataContainerERT, Mesh, create_box_mesh_3d
+from pygimli_gb300.data import geometricFactors, grid_line_scheme
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-8
+
+
+@pytest.fixture(scope="module")
+def torch():
+    t = pytest.importorskip("torch")
+    if not t.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from pygimli_gb300 import build
+    build.build()
+    return t
+
+
+def box(nx=5, ny=3, h=2.0, **kw):
+    e = np.array([(x, y) for x in np.arange(nx) * 4.0 for y in np.arange(ny) * 4.0])
+    mesh = create_box_mesh_3d(e, h=h, para_depth=10.0, outer=120.0, growth=1.5, **kw)
+    data = DataContainerERT(np.column_stack([e, np.zeros(len(e))]), grid_line_scheme((nx, ny), "pd"))
+    data.set("k", geometricFactors(data, 3))
+    return mesh, data
+
+
+def ground(mesh, kind, seed=1):
+    rng = np.random.default_rng(seed)
+    if kind == "homogeneous":
+        return np.full(mesh.cellCount(), 100.0)
+    rho = np.exp(rng.normal(np.log(100.0), 1.0, mesh.cellCount()))
+    if kind == "contrast":  # a conductor and an insulator, 1e5 apart
+        c = mesh.cellCenters()
+        rho[np.linalg.norm(c - [6.0, 4.0, -4.0], axis=1) < 3.0] = 0.3
+        rho[np.linalg.norm(c - [12.0, 4.0, -5.0], axis=1) < 3.0] = 3e4
+    return rho
+
+
+def operator(mesh, data, **kw):
+    from pygimli_gb300 import ERTModelling
+    f = ERTModelling(maxIter=200000, **kw)
+    f.setData(data)
+    f.setMesh(mesh, ignoreRegionManager=True)
+    return f
+
+
+def mixed(mesh, data, precond, **kw):
+    if precond == "learned":
+        import pygimli_gb300
+        kw["weights"] = os.path.join(os.path.dirname(pygimli_gb300.__file__), "weights", "box_3d.npz")
+    return operator(mesh, data, precision="mixed", precond=precond, **kw)
+
+
+def agree(fast, exact, rho):
+    r, r0 = fast.response(rho), exact.response(rho)
+    u, u0 = fast.subPotentials(), exact.subPotentials()
+    scale = np.maximum(np.abs(u0).max(axis=2), 1e-300)
+    e = float(np.max(np.abs(u - u0).max(axis=2) / scale))
+    assert e <= TOL, e
+    assert np.all(np.isfinite(r)) and float(np.max(np.abs(r - r0) / np.maximum(np.abs(r0), 1e-3))) <= 1e-5
+    st = fast.stats()
+    assert 0 < st["iterations"] <= 90 and st["stalled_columns"] == 0, st
+
+
+@pytest.mark.parametrize("kind", ["random", "contrast", "homogeneous"])
+@pytest.mark.parametrize("precond", ["jacobi", "fsai", "learned"])
+def test_smoothers(torch, precond, kind):
+    mesh, data = box()
+    assert mesh.nodeCount() >= 8192
+    fast, exact = mixed(mesh, data, precond), operator(mesh, data, rtol=1e-12)
+    for seed in (1, 2):  # the levels' patterns are kept, their values are not
+        agree(fast, exact, ground(mesh, kind, seed))
+
+
+@pytest.mark.parametrize("precond", ["jacobi", "fsai"])
+def test_quadratic_and_tight(torch, precond):
+    """P2 matrices (positive couplings, long rows) and rtol 1e-12."""
+    mesh, data = box(nx=4, ny=3, h=4.0)
+    mesh = mesh.createP2()
+    assert mesh.nodeCount() >= 8192
+    agree(mixed(mesh, data, precond, rtol=1e-12), operator(mesh, data, rtol=1e-12), ground(mesh, "random"))
+
+
+def with_markers(mesh, bm, nm=None):
+    return Mesh(3, mesh.nodes, mesh.cells, mesh.cell_markers, mesh.node_markers if nm is None else nm,
+                mesh.boundaries, bm, mesh.boundary_cells)
+
+
+@pytest.mark.parametrize("sr", [True, False])
+@pytest.mark.parametrize("where", ["sides", "all"])
+def test_dirichlet(torch, sr, where):
+    """Rows without couplings (homogeneous Dirichlet nodes) stay out of the
+    coarse levels."""
+    mesh, data = box()
+    bm = np.array(mesh.boundary_markers)
+    c = mesh.nodes[mesh.boundaries].mean(axis=1)
+    bm[(bm == -2) & ((c[:, 2] > c[:, 2].min() + 1e-6) | (where == "all"))] = -3
+    m = with_markers(mesh, bm)
+    agree(mixed(m, data, "fsai", sr=sr), operator(m, data, rtol=1e-12, sr=sr), ground(m, "random"))
+
+
+def test_closed_domain(torch):
+    """Neumann-only domain: a calibration node and the last electrode as the
+    reference; the levels follow a changed set of fixed rows."""
+    mesh, data = box()
+    data.set("k", np.ones(data.size()))
+    bm = np.array(mesh.boundary_markers)
+    bm[bm == -2] = -1
+    nm = np.array(mesh.node_markers)
+    fast = None
+    for calib in (0, 4321):
+        n2 = nm.copy()
+        n2[calib] = -1000
+        m = with_markers(mesh, bm, n2)
+        if fast is None:
+            fast = mixed(m, data, "fsai", sr=False)
+        else:
+            fast.setMesh(m, ignoreRegionManager=True)
+        agree(fast, operator(m, data, rtol=1e-12, sr=False), ground(m, "random"))
+
+
+def test_cem(torch):
+    from pygimli_gb300.cem import mark_cem_electrodes
+    mesh, data = box()
+    m = mark_cem_electrodes(mesh, data.sensorPositions()[:, :2], 2.0 * np.sqrt(2.0) * (1.0 + 1e-6))
+    agree(mixed(m, data, "fsai", sr=False), operator(m, data, rtol=1e-12, sr=False), ground(m, "random"))
