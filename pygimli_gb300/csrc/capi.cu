@@ -188,6 +188,7 @@ void ensure_derived(Context &c) {
         if (total) c.d_S1.release();  // the unit-resistivity matrix only serves singularity removal
         else assemble_unit(c, c.stream);
         c.s1_ready = true;
+        c.pnorm_ready = false;
     }
 }
 
@@ -226,7 +227,7 @@ int do_response(Context &c, const double *rho, double *rhoa, void *stream) {
         build_rhs_total(c, s);
     } else {
         build_rhs(c, s);
-        compute_rhs_scale(c, s);
+        if (c.precond != ERTGB_PRECOND_BAND) compute_rhs_scale(c, s);  // the direct solve has no convergence test
     }
     ERTGB_CUDA(cudaEventRecord(c.ev[2], s));
     c.have_S = true;
