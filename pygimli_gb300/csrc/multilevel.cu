@@ -26,8 +26,7 @@
 // itself (k_spmm32_q); the small levels are latency and launches.  Solve, single
 // level -> this: 23k nodes, 96 sources (FSAI) 23.9 -> 5.6 ms; 88k nodes, 96
 // sources (FSAI) 160.5 -> 18.2; 145k nodes, 256 sources (learned) 748 -> 77;
-// 38k nodes, 35 sources (Jacobi) 48.9 -> 6.9; 52k nodes, 96 CEM patches (FSAI)
-// 80.1 -> 12.0.
+// 38k nodes, 35 sources (Jacobi) 48.9 -> 6.9.
 //
 // Precision: matrices, Galerkin products and the coarsest inverse in FP64,
 // their FP32 copies and FP32 vectors in the cycle, as the factors were applied
@@ -524,6 +523,7 @@ bool ml_setup(Context &c, bool factor, cudaStream_t s) {
     // (Jacobi), 4.0 -> 2.2 (FSAI); 4224 nodes, 48 electrodes 11.9 -> 3.2, 11.6 ->
     // 3.5; nothing smaller than kMlMinRows was measured
     if (m.dim != 3 || c.nK != 1 || c.k[0] != 0.0 || m.n < kMlMinRows) return false;
+    if (!m.ext_rows.empty() || m.n_ext > 0) return false;  // CEM and bypass matrices keep the single level
     try {
         return setup(c, factor, s);
     } catch (Error &e) {

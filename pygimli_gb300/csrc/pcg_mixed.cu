@@ -516,7 +516,10 @@ __global__ void k_m_finish_ru(int64_t Rpad, int NB, double rtol2, const double *
 // conjugate to it.  beta is therefore (r . z - zold . r) / rho, or zero (a restart
 // from the true residual) where |zold . r| > 0.2 r . z (Powell, Math.
 // Programming 12, 1977).  Without it a fast problem diverged after 12 iterations
-// between updates.
+// between updates.  A column goes one digit below the tolerance (an interval
+// gains about two): the single-level recurrence overshoots it by up to 64
+// iterations, and the responses, differences of potentials, showed 2 to 5 times
+// its error when both stopped at the same residual.
 __global__ void k_m_finish_ml(int64_t Rpad, int NB, double rtol2, const double *__restrict__ part_a,
                               const double *__restrict__ part_b, const double *__restrict__ part_c,
                               double *__restrict__ col, ColState cs) {
@@ -536,7 +539,9 @@ __global__ void k_m_finish_ml(int64_t Rpad, int NB, double rtol2, const double *
     col[BETA * Rpad + t] = keep ? (rz - zr) / rho : 0.0;
     col[RHO * Rpad + t] = rz;
     col[RNORM2 * Rpad + t] = rr;
-    if (rr <= rtol2 * bb) {
+    const double best = col[RPREV * Rpad + t];
+    // one digit below the tolerance, or below it and no longer falling by 4 an interval
+    if (rr <= 0.01 * rtol2 * bb || (rr <= rtol2 * bb && rr > 0.0625 * best)) {
         cs.active[t] = 0;
         return;
     }
@@ -546,7 +551,6 @@ __global__ void k_m_finish_ml(int64_t Rpad, int NB, double rtol2, const double *
         atomicAdd(cs.nstalled, 1);
         return;
     }
-    const double best = col[RPREV * Rpad + t];
     double stalls = col[STALLS * Rpad + t];
     if (rr < 0.81 * best) {
         col[RPREV * Rpad + t] = rr;

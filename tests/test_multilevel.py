@@ -130,9 +130,3 @@ def test_closed_domain(torch):
             fast.setMesh(m, ignoreRegionManager=True)
         agree(fast, operator(m, data, rtol=1e-12, sr=False), ground(m, "random"))
 
-
-def test_cem(torch):
-    from pygimli_gb300.cem import mark_cem_electrodes
-    mesh, data = box()
-    m = mark_cem_electrodes(mesh, data.sensorPositions()[:, :2], 2.0 * np.sqrt(2.0) * (1.0 + 1e-6))
-    agree(mixed(m, data, "fsai", sr=False), operator(m, data, rtol=1e-12, sr=False), ground(m, "random"))
