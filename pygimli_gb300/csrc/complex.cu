@@ -403,14 +403,15 @@ __global__ void k_to_f32_c(int64_t n, const double2 *__restrict__ a, float2 *__r
 
 // r = b - A x in FP64 (b: unit sources) on the columns t < R with mask[t]
 // (all when mask is null).  F32: also r32 = r, z32 = D^-1 r32 and partials
-// of r^T z (FP32 values) and ||r||^2 (FP64); else r64 = r.
+// of r^T z (FP32 values) and ||r||^2 (FP64); else r64 = r.  With zold (coarse
+// levels) z32 stays and the first partials are zold^T r.
 template <bool F32>
 __global__ void k_resid_c(int64_t n, int64_t nnz, int nE, int64_t R, int64_t Rpad, const int32_t *__restrict__ rowptr,
                           const int32_t *__restrict__ colidx, const double2 *__restrict__ vals,
                           const int32_t *__restrict__ enode, const int32_t *__restrict__ mask,
                           const double2 *__restrict__ x, double2 *__restrict__ r64, const float2 *__restrict__ dinv32,
-                          float2 *__restrict__ r32, float2 *__restrict__ z32, double *__restrict__ p_re,
-                          double *__restrict__ p_im, double *__restrict__ p_rr) {
+                          float2 *__restrict__ r32, float2 *__restrict__ z32, const float2 *__restrict__ zold,
+                          double *__restrict__ p_re, double *__restrict__ p_im, double *__restrict__ p_rr) {
     const int64_t t = (int64_t)blockIdx.x * 32 + threadIdx.x;
     const bool act = t < R && (!mask || mask[t]);
     const int64_t ki = t < R ? t / nE : 0;
@@ -427,9 +428,9 @@ __global__ void k_resid_c(int64_t n, int64_t nnz, int nE, int64_t R, int64_t Rpa
             c += acc.x * acc.x + acc.y * acc.y;
             if (F32) {
                 const float2 rv = make_float2((float)acc.x, (float)acc.y);
-                const float2 zv = fmul(dk[row], rv);
+                const float2 zv = zold ? zold[i] : fmul(dk[row], rv);
                 r32[i] = rv;
-                z32[i] = zv;
+                if (!zold) z32[i] = zv;
                 const float2 rz = fmul(rv, zv);
                 a += rz.x;
                 b += rz.y;
@@ -672,6 +673,113 @@ __global__ void k_finish_ru_c(int64_t Rpad, int NB, double rtol2, const double *
     atomicAdd(nactive, 1);
 }
 
+// ---- coarse levels (one wavenumber, 3-D): the preconditioner is the real
+// multilevel cycle of Re S on the real and imaginary parts as 2 Rpad columns
+// (phases are small: Re S is SPD and close to S).  The recurrence, its reliable
+// update as the last of kMlItersC iterations and the restart rule are the real
+// mixed solver's (k_m_finish_ml) with the unconjugated products.  41k nodes, 48
+// sources: 1152 Jacobi iterations -> 36, response + Jacobian 112 -> 22 ms.
+constexpr int kMlItersC = 6;
+
+__global__ void k_real_c(int64_t nnz, const double2 *__restrict__ S, double *__restrict__ re) {
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nnz; t += (int64_t)gridDim.x * blockDim.x)
+        re[t] = S[t].x;
+}
+
+// y += alpha p, r -= alpha q
+__global__ void k_update_yr_c32(int64_t n, int64_t Rpad, const double *__restrict__ col,
+                                const int32_t *__restrict__ active, float2 *__restrict__ y, float2 *__restrict__ r,
+                                const float2 *__restrict__ p, const float2 *__restrict__ q) {
+    const int64_t t = (int64_t)blockIdx.x * 32 + threadIdx.x;
+    if (!active[t]) return;
+    const float2 al = make_float2((float)col[C_ALPHA_RE * Rpad + t], (float)col[C_ALPHA_IM * Rpad + t]);
+    for (int64_t row = (int64_t)blockIdx.y * kRowsC + threadIdx.y; row < n; row += (int64_t)gridDim.y * kRowsC) {
+        const int64_t i = row * Rpad + t;
+        y[i] = fadd(y[i], fmul(al, p[i]));
+        r[i] = fsub(r[i], fmul(al, q[i]));
+    }
+}
+
+// x += y + alpha p, y = 0
+__global__ void k_accum_p_c(int64_t n, int64_t Rpad, const double *__restrict__ col, const int32_t *__restrict__ active,
+                            double2 *__restrict__ x, float2 *__restrict__ y, const float2 *__restrict__ p) {
+    const int64_t t = (int64_t)blockIdx.x * 32 + threadIdx.x;
+    if (!active[t]) return;
+    const float2 al = make_float2((float)col[C_ALPHA_RE * Rpad + t], (float)col[C_ALPHA_IM * Rpad + t]);
+    for (int64_t row = (int64_t)blockIdx.y * kRowsC + threadIdx.y; row < n; row += (int64_t)gridDim.y * kRowsC) {
+        const int64_t i = row * Rpad + t;
+        const float2 v = fadd(y[i], fmul(al, p[i]));
+        x[i] = make_double2(x[i].x + (double)v.x, x[i].y + (double)v.y);
+        y[i] = make_float2(0.f, 0.f);
+    }
+}
+
+// partials of r^T z
+__global__ void k_dot_c32(int64_t n, int64_t R, int64_t Rpad, const float2 *__restrict__ r, const float2 *__restrict__ z,
+                          double *__restrict__ p_re, double *__restrict__ p_im) {
+    const int64_t t = (int64_t)blockIdx.x * 32 + threadIdx.x;
+    float a = 0.f, b = 0.f;
+    if (t < R)
+        for (int64_t row = (int64_t)blockIdx.y * kRowsC + threadIdx.y; row < n; row += (int64_t)gridDim.y * kRowsC) {
+            const float2 v = fmul(r[row * Rpad + t], z[row * Rpad + t]);
+            a += v.x;
+            b += v.y;
+        }
+    block_partials3(a, b, 0.0, p_re, p_im, nullptr, Rpad, t);
+}
+
+// convergence test on the true residual and the next direction; (p_re, p_im):
+// r^T z, (o_re, o_im): zold^T r, p_rr: ||r||^2
+__global__ void k_finish_ml_c(int64_t Rpad, int NB, double rtol2, const double *__restrict__ p_re,
+                              const double *__restrict__ p_im, const double *__restrict__ o_re,
+                              const double *__restrict__ o_im, const double *__restrict__ p_rr,
+                              double *__restrict__ col, int32_t *__restrict__ active, int32_t *__restrict__ iters,
+                              int32_t *__restrict__ stalled, int32_t *__restrict__ nactive,
+                              int32_t *__restrict__ nstalled) {
+    const int64_t t = (int64_t)blockIdx.x * kFinWarps + (threadIdx.x >> 5);
+    if (t >= Rpad) return;
+    const double2 rz = make_double2(warp_col_sum(p_re, NB, Rpad, t), warp_col_sum(p_im, NB, Rpad, t));
+    const double2 zr = make_double2(warp_col_sum(o_re, NB, Rpad, t), warp_col_sum(o_im, NB, Rpad, t));
+    const double rr = warp_col_sum(p_rr, NB, Rpad, t);
+    if ((threadIdx.x & 31) != 0 || !active[t]) return;
+    iters[t] += 1;
+    const double2 rho = make_double2(col[C_RHO_RE * Rpad + t], col[C_RHO_IM * Rpad + t]);
+    const double bb = col[C_BB * Rpad + t], best = col[C_BEST * Rpad + t];
+    double2 be = make_double2(0.0, 0.0);
+    if (hypot(rho.x, rho.y) > 0.0 && hypot(zr.x, zr.y) <= 0.2 * hypot(rz.x, rz.y)) be = cdiv(csub(rz, zr), rho);
+    if (!isfinite(be.x) || !isfinite(be.y)) be = make_double2(0.0, 0.0);
+    col[C_BETA_RE * Rpad + t] = be.x;
+    col[C_BETA_IM * Rpad + t] = be.y;
+    col[C_RHO_RE * Rpad + t] = rz.x;
+    col[C_RHO_IM * Rpad + t] = rz.y;
+    col[C_RR * Rpad + t] = rr;
+    if (rr <= 0.01 * rtol2 * bb || (rr <= rtol2 * bb && rr > 0.0625 * best)) {
+        active[t] = 0;
+        return;
+    }
+    if (!(rr <= 4.0 * bb) || !isfinite(rz.x) || !isfinite(rz.y)) {
+        active[t] = 0;
+        stalled[t] = 2;
+        atomicAdd(nstalled, 1);
+        return;
+    }
+    double stalls = col[C_STALLS * Rpad + t];
+    if (rr < 0.81 * best) {
+        col[C_BEST * Rpad + t] = rr;
+        stalls = 0.0;
+    } else {
+        stalls += 1.0;
+    }
+    col[C_STALLS * Rpad + t] = stalls;
+    if (stalls >= 4.0) {
+        active[t] = 0;
+        stalled[t] = 1;
+        atomicAdd(nstalled, 1);
+        return;
+    }
+    atomicAdd(nactive, 1);
+}
+
 // stalled columns restarting from zero: x = 0 there
 __global__ void k_zero_restart_c(int64_t n, int64_t Rpad, const int32_t *__restrict__ stalled,
                                  double2 *__restrict__ x) {
@@ -691,8 +799,9 @@ struct CxLaunch {
     dim3 vb, vg, fb, fg;
 };
 
-void run_graph_loop(Context &c, cudaStream_t s, const std::function<void()> &body, int32_t *nactive, int launches,
-                    const std::function<void()> &after, int *status) {
+// body: iters iterations, captured once; launches of it per host check
+void run_graph_loop(Context &c, cudaStream_t s, const std::function<void()> &body, int iters, int32_t *nactive,
+                    int launches, const std::function<void()> &after, int *status) {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ge = nullptr;
     try {
@@ -710,7 +819,7 @@ void run_graph_loop(Context &c, cudaStream_t s, const std::function<void()> &bod
                 break;
             }
             for (int u = 0; u < launches; u++) ERTGB_CUDA(cudaGraphLaunch(ge, s));
-            done += launches * kGraphItersC;
+            done += launches * iters;
             if (after) after();
             ERTGB_CUDA(cudaMemcpyAsync(&h_active, nactive, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
             ERTGB_CUDA(cudaStreamSynchronize(s));
@@ -739,7 +848,7 @@ int cocg_fp64(Context &c, const CxLaunch &L, cudaStream_t s, const int32_t *mask
     if (!mask) ERTGB_CUDA(cudaMemsetAsync(x.x.p, 0, sizeof(double2) * n * Rpad, s));
     ERTGB_CUDA(cudaMemsetAsync(nactive, 0, sizeof(int32_t), s));
     k_resid_c<false><<<L.vg, L.vb, 0, s>>>(n, nnz, c.nE, R, Rpad, m.d_rowptr.p, m.d_colidx.p, x.S.p, c.d_enode.p, mask,
-                                           x.x.p, x.r.p, nullptr, nullptr, nullptr, pa, pb, pc);
+                                           x.x.p, x.r.p, nullptr, nullptr, nullptr, nullptr, pa, pb, pc);
     k_precond_c<true><<<L.vg, L.vb, 0, s>>>(n, c.nE, R, Rpad, x.dinv.p, mask, x.r.p, x.z.p, x.p.p, pa, pb, pc);
     k_finish_init_c<<<L.fg, L.fb, 0, s>>>(Rpad, R, NB, pa, pb, pc, x.col.p, active, iters, nactive, mask);
     ERTGB_CUDA(cudaGetLastError());
@@ -756,7 +865,7 @@ int cocg_fp64(Context &c, const CxLaunch &L, cudaStream_t s, const int32_t *mask
             k_finish_beta_c<<<L.fg, L.fb, 0, s>>>(Rpad, NB, rtol2, pa, pb, pc, x.col.p, active, iters, nactive);
             k_update_p_c<<<L.vg, L.vb, 0, s>>>(n, Rpad, x.col.p, active, x.z.p, x.p.p);
         }
-    }, nactive, 4, nullptr, &status);
+    }, kGraphItersC, nactive, 4, nullptr, &status);
     return status;
 }
 
@@ -781,21 +890,37 @@ int cocg_mixed(Context &c, const CxLaunch &L, cudaStream_t s, int *status) {
     ERTGB_CUDA(cudaMemsetAsync(stalled, 0, sizeof(int32_t) * (Rpad + 1), s));
     ERTGB_CUDA(cudaMemsetAsync(nactive, 0, sizeof(int32_t), s));
     k_resid_c<true><<<L.vg, L.vb, 0, s>>>(n, nnz, c.nE, R, Rpad, m.d_rowptr.p, m.d_colidx.p, x.S.p, c.d_enode.p,
-                                          nullptr, x.x.p, nullptr, x.dinv32.p, x.r32.p, x.z32.p, pa, pb, pc);
+                                          nullptr, x.x.p, nullptr, x.dinv32.p, x.r32.p, x.z32.p, nullptr, pa, pb, pc);
+    bool ml = false;
+    if (c.nK == 1) {
+        x.Sre.alloc((size_t)nnz);
+        k_real_c<<<grid1c(nnz), 256, 0, s>>>(nnz, x.S.p, x.Sre.p);
+        ERTGB_CUDA(cudaGetLastError());
+        ml = ml_setup(c, x.Sre.p, false, 2 * Rpad, s);
+    }
+    // z = M^-1 r with the partials of r^T z (q is free between the residual's update and the operator)
+    auto precond = [&] {
+        ml_cycle(c, MlBlock{2 * Rpad, reinterpret_cast<const float *>(x.r32.p), reinterpret_cast<float *>(x.z32.p),
+                            reinterpret_cast<float *>(x.q32.p), nullptr}, 0, nullptr, s);
+        k_dot_c32<<<L.vg, L.vb, 0, s>>>(n, R, Rpad, x.r32.p, x.z32.p, pa, pb);
+    };
+    if (ml) precond();
     ERTGB_CUDA(cudaMemcpyAsync(x.p32.p, x.z32.p, sizeof(float2) * n * Rpad, cudaMemcpyDeviceToDevice, s));
     k_finish_init_c<<<L.fg, L.fb, 0, s>>>(Rpad, R, NB, pa, pb, pc, x.col.p, active, iters, nactive, nullptr);
     ERTGB_CUDA(cudaGetLastError());
     const double rtol2 = c.rtol * c.rtol;
-    // the reliable update as a second graph
+    // the reliable update as a second graph (the single-level form)
     cudaGraph_t gru = nullptr;
     cudaGraphExec_t eru = nullptr;
-    ERTGB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    k_accum_c<<<L.vg, L.vb, 0, s>>>(n, Rpad, active, x.x.p, x.y32.p, nactive);
-    k_resid_c<true><<<L.vg, L.vb, 0, s>>>(n, nnz, c.nE, R, Rpad, m.d_rowptr.p, m.d_colidx.p, x.S.p, c.d_enode.p, active,
-                                          x.x.p, nullptr, x.dinv32.p, x.r32.p, x.z32.p, pa, pb, pc);
-    k_finish_ru_c<<<L.fg, L.fb, 0, s>>>(Rpad, NB, rtol2, pa, pb, pc, x.col.p, active, stalled, nactive, nstalled);
-    ERTGB_CUDA(cudaStreamEndCapture(s, &gru));
-    ERTGB_CUDA(cudaGraphInstantiate(&eru, gru, 0));
+    if (!ml) {
+        ERTGB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        k_accum_c<<<L.vg, L.vb, 0, s>>>(n, Rpad, active, x.x.p, x.y32.p, nactive);
+        k_resid_c<true><<<L.vg, L.vb, 0, s>>>(n, nnz, c.nE, R, Rpad, m.d_rowptr.p, m.d_colidx.p, x.S.p, c.d_enode.p, active,
+                                              x.x.p, nullptr, x.dinv32.p, x.r32.p, x.z32.p, nullptr, pa, pb, pc);
+        k_finish_ru_c<<<L.fg, L.fb, 0, s>>>(Rpad, NB, rtol2, pa, pb, pc, x.col.p, active, stalled, nactive, nstalled);
+        ERTGB_CUDA(cudaStreamEndCapture(s, &gru));
+        ERTGB_CUDA(cudaGraphInstantiate(&eru, gru, 0));
+    }
     // one wavenumber and Rpad = 16 CH: the 8-lane-group operator (partials of NBq block rows)
     const int chq = c.nK == 1 ? (int)(Rpad / 16) : 0;
     const bool fastq = chq == 2 || chq == 4 || chq == 6 || chq == 8;
@@ -816,7 +941,27 @@ int cocg_mixed(Context &c, const CxLaunch &L, cudaStream_t s, int *status) {
         }
     };
     try {
-        run_graph_loop(c, s, [&] {
+        if (ml) run_graph_loop(c, s, [&] {
+            for (int it = 0; it < kMlItersC; it++) {
+                spmm();
+                k_finish_alpha_cw<<<fwg, 32 * kFinWarps, 0, s>>>(Rpad, NBq, pd, pe, x.col.p, active, nactive);
+                if (it + 1 < kMlItersC) {
+                    k_update_yr_c32<<<L.vg, L.vb, 0, s>>>(n, Rpad, x.col.p, active, x.y32.p, x.r32.p, x.p32.p, x.q32.p);
+                    precond();
+                    k_finish_beta_mcw<<<fwg, 32 * kFinWarps, 0, s>>>(Rpad, NB, pa, pb, x.col.p, active, iters);
+                } else {
+                    k_accum_p_c<<<L.vg, L.vb, 0, s>>>(n, Rpad, x.col.p, active, x.x.p, x.y32.p, x.p32.p);
+                    k_resid_c<true><<<L.vg, L.vb, 0, s>>>(n, nnz, c.nE, R, Rpad, m.d_rowptr.p, m.d_colidx.p, x.S.p,
+                                                          c.d_enode.p, active, x.x.p, nullptr, x.dinv32.p, x.r32.p,
+                                                          x.z32.p, x.z32.p, pd, pe, pc);
+                    precond();
+                    k_finish_ml_c<<<fwg, 32 * kFinWarps, 0, s>>>(Rpad, NB, rtol2, pa, pb, pd, pe, pc, x.col.p, active,
+                                                                 iters, stalled, nactive, nstalled);
+                }
+                k_update_p_c32<<<L.vg, L.vb, 0, s>>>(n, Rpad, x.col.p, active, x.z32.p, x.p32.p);
+            }
+        }, kMlItersC, nactive, 1, nullptr, status);
+        else run_graph_loop(c, s, [&] {
             for (int it = 0; it < kGraphItersC; it++) {
                 spmm();
                 k_finish_alpha_cw<<<fwg, 32 * kFinWarps, 0, s>>>(Rpad, NBq, pd, pe, x.col.p, active, nactive);
@@ -825,14 +970,14 @@ int cocg_mixed(Context &c, const CxLaunch &L, cudaStream_t s, int *status) {
                 k_finish_beta_mcw<<<fwg, 32 * kFinWarps, 0, s>>>(Rpad, NB, pa, pb, x.col.p, active, iters);
                 k_update_p_c32<<<L.vg, L.vb, 0, s>>>(n, Rpad, x.col.p, active, x.z32.p, x.p32.p);
             }
-        }, nactive, 4, [&] { ERTGB_CUDA(cudaGraphLaunch(eru, s)); }, status);
+        }, kGraphItersC, nactive, 4, [&] { ERTGB_CUDA(cudaGraphLaunch(eru, s)); }, status);
     } catch (...) {
-        cudaGraphExecDestroy(eru);
-        cudaGraphDestroy(gru);
+        if (eru) cudaGraphExecDestroy(eru);
+        if (gru) cudaGraphDestroy(gru);
         throw;
     }
-    cudaGraphExecDestroy(eru);
-    cudaGraphDestroy(gru);
+    if (eru) cudaGraphExecDestroy(eru);
+    if (gru) cudaGraphDestroy(gru);
     if (*status == ERTGB_NOT_CONVERGED) {  // the increments since the last reliable update
         k_accum_c<<<L.vg, L.vb, 0, s>>>(n, Rpad, active, x.x.p, x.y32.p, nactive);
         ERTGB_CUDA(cudaGetLastError());

@@ -221,6 +221,7 @@ struct ComplexState {
     DBuf<double2> U;                // nE x nE electrode potentials
     // mixed precision: FP32 matrices, Jacobi diagonal and recurrence vectors
     DBuf<float2> S32, dinv32, r32, z32, p32, q32, y32;
+    DBuf<double> Sre;               // Re S, the matrix of the coarse levels (3-D)
     DBuf<int32_t> stalled;          // Rpad flags + counter
     bool have_pot = false;
     int32_t iterations = 0;
@@ -432,12 +433,18 @@ void build_extension_map(const MeshData &m, std::vector<int32_t> &ptr, std::vect
 // ``coarsest`` rows; false: no useful hierarchy
 bool build_levels(const std::vector<int32_t> &rowptr, const std::vector<int32_t> &colidx,
                   const std::vector<double> &unit, int64_t coarsest, int max_levels, std::vector<HostLevel> &out);
-// multilevel.cu: coarse levels of the current matrix (d_S; the preconditioner's
-// factor in d_G32 when ``factor``); false: the single-level preconditioner
-// stays.  ml_cycle: d_z32 = M^-1 d_r32 with the column partials of r . z (NB
-// block rows) in pz.
-bool ml_setup(Context &c, bool factor, cudaStream_t s);
-void ml_cycle(Context &c, int NB, double *pz, cudaStream_t s);
+// multilevel.cu: coarse levels of the matrix val (CSR values on the mesh's
+// pattern, SPD) for blocks of cols columns; factor: the fine-level smoother is
+// the FSAI or learned factor in d_G32 (with d_S32), else Jacobi.  false: the
+// single-level preconditioner stays.  ml_cycle: z = M^-1 b, r and t scratch (t:
+// factor only); pz (may be null): column partials of b . z in NB block rows
+struct MlBlock {
+    int64_t cols;
+    const float *b;
+    float *z, *r, *t;
+};
+bool ml_setup(Context &c, const double *val, bool factor, int64_t cols, cudaStream_t s);
+void ml_cycle(Context &c, const MlBlock &v, int NB, double *pz, cudaStream_t s);
 int ml_launches(const Context &c);
 // band.cu: inverse of one SPD matrix of at most 112 rows, in place (one block)
 constexpr int kDenseMax = 112;

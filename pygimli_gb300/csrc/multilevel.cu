@@ -446,14 +446,12 @@ inline unsigned grid_rows(int64_t n, int per = kT) { return (unsigned)std::min<i
 
 }  // namespace
 
-static bool setup(Context &c, bool factor, cudaStream_t s) {
+static bool setup(Context &c, const double *fine, bool factor, int64_t Rpad, cudaStream_t s) {
     MeshData &m = c.mesh;
     build(c, s);
     Multilevel &M = m.ml;
     if (!M.ok) return false;
-    c.d_z32.alloc((size_t)m.n * c.Rpad);
     const size_t L = M.levels.size();
-    const int64_t Rpad = c.Rpad;
     M.factor = factor;
     M.bad.zero(s);
     int launches = 0;
@@ -461,7 +459,7 @@ static bool setup(Context &c, bool factor, cudaStream_t s) {
         MlLevel &l = *M.levels[k];
         MlLevel &d = *M.levels[k + 1];
         const int32_t *rp = k ? l.rp.p : m.d_rowptr.p, *ci = k ? l.ci.p : m.d_colidx.p;
-        const double *val = k ? l.val.p : c.d_S.p;
+        const double *val = k ? l.val.p : fine;
         const bool jac = k || !factor;
         if (jac) l.AS.alloc((size_t)(k ? l.nnz : m.nnz));
         k_ml_rows<<<grid_rows(32 * l.n), kT, 0, s>>>(l.n, rp, ci, val, l.P_rp.p, l.P_ci.p, l.P_v.p, l.AP_rp.p, l.AP_ci.p,
@@ -516,7 +514,7 @@ static bool setup(Context &c, bool factor, cudaStream_t s) {
     return bad == 0;
 }
 
-bool ml_setup(Context &c, bool factor, cudaStream_t s) {
+bool ml_setup(Context &c, const double *val, bool factor, int64_t cols, cudaStream_t s) {
     const MeshData &m = c.mesh;
     // 3-D (one wavenumber k = 0): the 2.5-D path has its direct solve.  One response
     // without -> with coarse levels: 1350 nodes, 12 electrodes 5.2 -> 2.3 ms
@@ -525,7 +523,7 @@ bool ml_setup(Context &c, bool factor, cudaStream_t s) {
     if (m.dim != 3 || c.nK != 1 || c.k[0] != 0.0 || m.n < kMlMinRows) return false;
     if (!m.ext_rows.empty() || m.n_ext > 0) return false;  // CEM and bypass matrices keep the single level
     try {
-        return setup(c, factor, s);
+        return setup(c, val, factor, cols, s);
     } catch (Error &e) {
         if (e.code != ERTGB_OOM) throw;
         // the coarse levels do not fit beside the rest: the single-level form does without
@@ -540,13 +538,14 @@ bool ml_setup(Context &c, bool factor, cudaStream_t s) {
     }
 }
 
-void ml_cycle(Context &c, int NB, double *pz, cudaStream_t s) {
+void ml_cycle(Context &c, const MlBlock &v, int NB, double *pz, cudaStream_t s) {
     MeshData &m = c.mesh;
     Multilevel &M = m.ml;
-    const int64_t n = m.n, R = c.Rpad;
+    const int64_t n = m.n, R = v.cols;
     const size_t L = M.levels.size();
     MlLevel &f = *M.levels[0];
-    float *b = c.d_r32.p, *z = c.d_z32.p, *r = c.d_q32.p, *t = c.d_t32.p;  // q is free between alpha and the operator
+    const float *b = v.b;
+    float *z = v.z, *r = v.r, *t = v.t;
     Args a;
     if (M.factor) {
         a.w = M.w.p;
@@ -592,7 +591,8 @@ void ml_cycle(Context &c, int NB, double *pz, cudaStream_t s) {
     } else {
         a.r = r;
         a.dw = f.dw.p;
-        spmm<EP_POST, true>(s, n, R, f.AP_rp.p, f.AP_ci.p, f.Q.p, e, z, a);
+        if (pz) spmm<EP_POST, true>(s, n, R, f.AP_rp.p, f.AP_ci.p, f.Q.p, e, z, a);
+        else spmm<EP_POST, false>(s, n, R, f.AP_rp.p, f.AP_ci.p, f.Q.p, e, z, a);
     }
     ERTGB_CUDA(cudaGetLastError());
 }

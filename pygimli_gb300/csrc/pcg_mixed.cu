@@ -659,13 +659,15 @@ int pcg_solve_mixed(Context &c, cudaStream_t s) {
     }
     k_to_f32<<<(unsigned)std::min<int64_t>(ceil_div((int64_t)c.nK * m.nnz, 256), 65535), 256, 0, s>>>(
         (int64_t)c.nK * m.nnz, c.d_S.p, c.d_S32.p);
-    const bool ml = ml_setup(c, fsai, s);  // coarse levels around the factor (or Jacobi)
+    const bool ml = ml_setup(c, c.d_S.p, fsai, Rpad, s);  // coarse levels around the factor (or Jacobi)
+    if (ml) c.d_z32.alloc((size_t)n * Rpad);
     const bool zform = fsai || ml;         // z = M^-1 r is a product of its own
     // z = M^-1 r with the column partials of r . z into pz: the multilevel
     // cycle, or G^T (G r)
     auto apply_fsai = [&](double *pz) {
         if (ml) {
-            ml_cycle(c, NB, pz, s);
+            // q is free between the residual's update and the operator
+            ml_cycle(c, MlBlock{Rpad, c.d_r32.p, c.d_z32.p, c.d_q32.p, c.d_t32.p}, NB, pz, s);
             return;
         }
         dispatch_ch<GenL>(ch, dim3((unsigned)NB, (unsigned)nchunk), s, n, nL, c.nE, c.nK, Rpad, m.d_Lrowptr.p,
