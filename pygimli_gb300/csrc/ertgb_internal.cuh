@@ -152,6 +152,7 @@ struct MeshData {
     // parameter -> cells (sorted by parameter), for the Jacobian
     std::vector<int32_t> pcell_ptr, pcell;
     DBuf<int32_t> d_pcell_ptr, d_pcell;
+    bool one_cell = false;  // no parameter has more than one cell
 };
 
 // A contiguous range of data [d0, d1) with its own distinct current and

@@ -812,6 +812,8 @@ void build_jacobian_tiles(Context &c) {
     std::vector<int32_t> pos(m.pcell_ptr.begin(), m.pcell_ptr.end() - 1);
     for (int64_t i = 0; i < m.C; i++)
         if (m.marker[i] >= 0) m.pcell[pos[m.marker[i]]++] = (int32_t)i;
+    m.one_cell = true;
+    for (int64_t p = 0; p < P; p++) m.one_cell = m.one_cell && m.pcell_ptr[p + 1] - m.pcell_ptr[p] <= 1;
     m.d_pcell_ptr.upload(m.pcell_ptr, c.stream);
     m.d_pcell.upload(m.pcell, c.stream);
     for (int dt = 0; dt < 2; dt++) {
