@@ -631,6 +631,8 @@ def run_ours(args, world, rank, local):
         rho): CUDA events over ``n_steps`` steps after ``n_warm`` warm-up steps."""
         m_, d_, r_ = wl
         fop_p = ERTModelling(device=local, rtol=args.rtol, precision=precision, precond=precond, weights=weights_)
+        if (precision, precond) == ("fp64", "jacobi"):
+            fop_p.setCoarseLevels(False)  # the plain PCG of the metric
         fop_p.setData(d_)
         fop_p.setMesh(m_, ignoreRegionManager=True)
         Dp, Pp, Cp = d_.size(), fop_p.parameterCount, m_.cellCount()

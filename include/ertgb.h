@@ -228,6 +228,9 @@ int ertgb_set_solver(ertgb_ctx *ctx, double rtol, int max_iter, int precond);
 /* Solver arithmetic (ertgb_precision).  No counterpart in the reference,
  * whose direct solver is FP64. */
 int ertgb_set_precision(ertgb_ctx *ctx, int precision);
+/* Coarse levels of the iterative solvers on 3-D meshes (on by default): 0
+ * leaves the preconditioner alone on the fine level, the plain PCG. */
+int ertgb_set_coarse_levels(ertgb_ctx *ctx, int on);
 
 /* Forward response: DCMultiElectrodeModelling::response
  * (core/src/bert/dcfemmodelling.cpp:1085-1197) for a per-cell resistivity

@@ -746,6 +746,11 @@ int ertgb_set_precision(ertgb_ctx *ctx, int precision) {
     });
 }
 
+int ertgb_set_coarse_levels(ertgb_ctx *ctx, int on) {
+    Context *c = reinterpret_cast<Context *>(ctx);
+    return guard(c, [&] { c->coarse_levels = on != 0; });
+}
+
 int ertgb_response(ertgb_ctx *ctx, const double *rho_cell_dev, double *rhoa_dev, void *stream) {
     Context *c = reinterpret_cast<Context *>(ctx);
     int status = ERTGB_OK;

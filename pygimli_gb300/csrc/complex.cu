@@ -970,7 +970,7 @@ int cocg_mixed(Context &c, const CxLaunch &L, cudaStream_t s, int *status) {
     }
     // z = M^-1 r with the partials of r^T z (q is free between the residual's update and the operator)
     auto precond = [&] {
-        ml_cycle(c, MlBlock{2 * Rpad, reinterpret_cast<const float *>(x.r32.p), reinterpret_cast<float *>(x.z32.p),
+        ml_cycle(c, MlBlock<float>{2 * Rpad, reinterpret_cast<const float *>(x.r32.p), reinterpret_cast<float *>(x.z32.p),
                             reinterpret_cast<float *>(x.q32.p), nullptr}, 0, nullptr, s);
         k_dot_c32<<<L.vg, L.vb, 0, s>>>(n, R, Rpad, x.r32.p, x.z32.p, pa, pb);
     };

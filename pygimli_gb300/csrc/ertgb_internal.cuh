@@ -93,14 +93,24 @@ struct HostLevel {
 };
 
 // The same on the device (multilevel.cu) with the values of the current model
-// and the level's vectors.  Level 0 uses the mesh's pattern and matrix.
+// and the level's vectors in the cycle's precision.  Level 0 uses the mesh's
+// pattern and matrix.
+template <typename T> struct MlValues {
+    DBuf<T> AS, Q, dw;  // A diag(dw) (coarsest: the inverse); the post-smoothed prolongation or -A P; the rows' damping
+    DBuf<T> b, r, e;    // right-hand side, residual, correction: n x columns
+};
 struct MlLevel {
     int64_t n = 0, nc = 0, nnz = 0, nnzP = 0, nnzAP = 0;
     DBuf<int32_t> rp, ci, P_rp, P_ci, PT_rp, PT_ci, AP_rp, AP_ci;
     DBuf<float> P_v, PT_v;
-    DBuf<double> val, AP;   // FP64 matrix (levels >= 1) and A P
-    DBuf<float> AS, Q, dw;  // A diag(dw); the post-smoothed prolongation (or -A P); the rows' damping
-    DBuf<float> b, r, e;    // right-hand side, residual, correction: n x Rpad
+    DBuf<double> PT64;
+    DBuf<double> val, AP;  // FP64 matrix (levels >= 1) and A P
+    MlValues<float> v32;
+    MlValues<double> v64;
+    template <typename T> MlValues<T> &values() {
+        if constexpr (sizeof(T) == 4) return v32;
+        else return v64;
+    }
 };
 
 struct Multilevel {
@@ -108,7 +118,6 @@ struct Multilevel {
     std::vector<uint8_t> fixed;      // the fixed rows it was built with
     std::vector<std::unique_ptr<MlLevel>> levels;  // the coarsest last
     DBuf<double> inv64;              // coarsest inverse
-    DBuf<float> inv32;
     DBuf<int32_t> bad;
     bool factor = false;             // fine-level smoother: the factor G^T G (else Jacobi)
     DBuf<float> w, px, pt, pg;       // the factor's damping; power iteration vectors (n x 32)
@@ -300,6 +309,7 @@ struct Context {
     int max_iter = 20000;
     int precond = ERTGB_PRECOND_JACOBI;
     int precision = ERTGB_PRECISION_FP64;
+    bool coarse_levels = true;    // multilevel preconditioner where it applies (ertgb_set_coarse_levels)
     int rhs_align = 32;           // Rpad granularity (batches use 128)
     // derived per (mesh, electrodes, kw)
     int64_t R = 0, Rpad = 0;     // right-hand sides nK*nE, padded to 32
@@ -438,14 +448,17 @@ bool build_levels(const std::vector<int32_t> &rowptr, const std::vector<int32_t>
 // pattern, SPD) for blocks of cols columns; factor: the fine-level smoother is
 // the FSAI or learned factor in d_G32 (with d_S32), else Jacobi.  false: the
 // single-level preconditioner stays.  ml_cycle: z = M^-1 b, r and t scratch (t:
-// factor only); pz (may be null): column partials of b . z in NB block rows
-struct MlBlock {
+// factor only); pz (may be null without a factor): column partials of b . z in
+// NB block rows.  The FP32 cycle and, Jacobi only, the FP64 one.
+template <typename T> struct MlBlock {
     int64_t cols;
-    const float *b;
-    float *z, *r, *t;
+    const T *b;
+    T *z, *r, *t;
 };
 bool ml_setup(Context &c, const double *val, bool factor, int64_t cols, cudaStream_t s);
-void ml_cycle(Context &c, const MlBlock &v, int NB, double *pz, cudaStream_t s);
+void ml_cycle(Context &c, const MlBlock<float> &v, int NB, double *pz, cudaStream_t s);
+bool ml_setup64(Context &c, const double *val, int64_t cols, cudaStream_t s);
+void ml_cycle64(Context &c, const MlBlock<double> &v, int NB, double *pz, cudaStream_t s);
 int ml_launches(const Context &c);
 // band.cu: inverse of one SPD matrix of at most 112 rows, in place (one block)
 constexpr int kDenseMax = 112;

@@ -28,9 +28,11 @@
 // sources (FSAI) 160.5 -> 18.2; 145k nodes, 256 sources (learned) 748 -> 77;
 // 38k nodes, 35 sources (Jacobi) 48.9 -> 6.9.
 //
-// Precision: matrices, Galerkin products and the coarsest inverse in FP64,
-// their FP32 copies and FP32 vectors in the cycle, as the factors were applied
-// before; the recurrence's FP64 true residual decides convergence.
+// Precision: matrices, Galerkin products and the coarsest inverse in FP64.  The
+// mixed solver's cycle holds their FP32 copies and FP32 vectors, as its factors
+// were applied before (its FP64 true residual decides convergence); the FP64
+// solver's cycle is FP64 throughout (Jacobi levels; 23k nodes, 96 sources: 671
+// iterations -> 39, 78.5 -> 20.8 ms).
 #include <algorithm>
 #include <cmath>
 
@@ -66,11 +68,12 @@ __device__ __forceinline__ int32_t find_col(const int32_t *__restrict__ ci, int3
 //   dw_i = kOmega / sum_j |a_ij|  (a row without a positive diagonal or with a
 //     value that is not finite counts as bad),
 //   Q = P - diag(dw) A P  (Jacobi level) or Q = -A P (factor level).
+template <typename T>
 __global__ void k_ml_rows(int64_t n, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci,
                           const double *__restrict__ val, const int32_t *__restrict__ prp,
                           const int32_t *__restrict__ pci, const float *__restrict__ pv,
                           const int32_t *__restrict__ arp, const int32_t *__restrict__ aci, int jacobi,
-                          double *__restrict__ ap, float *__restrict__ dw, float *__restrict__ Q,
+                          double *__restrict__ ap, T *__restrict__ dw, T *__restrict__ Q,
                           int32_t *__restrict__ bad) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -86,7 +89,7 @@ __global__ void k_ml_rows(int64_t n, const int32_t *__restrict__ rp, const int32
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         diag = __any_sync(0xffffffffu, diag);
-        const float d = (float)(kOmega / sum);
+        const T d = (T)(kOmega / sum);
         if (lane == 0) {
             if (!diag || !isfinite(sum)) atomicAdd(bad, 1);
             dw[i] = d;
@@ -106,19 +109,20 @@ __global__ void k_ml_rows(int64_t n, const int32_t *__restrict__ rp, const int32
                 double e = 0.0;
                 for (int32_t p = p0; p < p1; p++)
                     if (pci[p] == J) e = (double)pv[p];
-                Q[q] = (float)(e - (double)d * acc);
+                Q[q] = (T)(e - (double)d * acc);
             } else {
-                Q[q] = (float)-acc;
+                Q[q] = (T)-acc;
             }
         }
     }
 }
 
 // AS = A diag(dw)
+template <typename T>
 __global__ void k_ml_scale(int64_t nnz, const int32_t *__restrict__ ci, const double *__restrict__ val,
-                           const float *__restrict__ dw, float *__restrict__ AS) {
+                           const T *__restrict__ dw, T *__restrict__ AS) {
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nnz; t += (int64_t)gridDim.x * blockDim.x)
-        AS[t] = (float)(val[t] * (double)dw[ci[t]]);
+        AS[t] = (T)(val[t] * (double)dw[ci[t]]);
 }
 
 // P^T (A P), one warp per coarse row: the fine rows in order, lanes over the
@@ -155,11 +159,11 @@ __global__ void k_ml_densify(int n, const int32_t *__restrict__ rp, const int32_
     }
 }
 
-__global__ void k_ml_inverse32(int n, const double *__restrict__ A, float *__restrict__ B) {
+template <typename T> __global__ void k_ml_symmetric(int n, const double *__restrict__ A, T *__restrict__ B) {
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < (int64_t)n * n;
          t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = t / n, j = t - i * n;
-        B[t] = (float)(0.5 * (A[t] + A[j * n + i]));
+        B[t] = (T)(0.5 * (A[t] + A[j * n + i]));
     }
 }
 
@@ -176,50 +180,62 @@ enum Ep {
     EP_ACC,    // y += B x
     EP_FINAL,  // y = w B x + P e
 };
+// four adjacent columns
+template <typename T> struct Four;
+template <> struct Four<float> { using V = float4; };
+struct alignas(32) Double4 { double x, y, z, w; };
+template <> struct Four<double> { using V = Double4; };
+__device__ __forceinline__ float4 load4(const float4 *p) { return __ldg(p); }
+__device__ __forceinline__ Double4 load4(const Double4 *p) {
+    const double2 a = __ldg(reinterpret_cast<const double2 *>(p)), b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
+    return {a.x, a.y, b.x, b.y};
+}
+
 // Operands of one product; unused ones stay null.
-struct Args {
-    const float *b = nullptr, *r = nullptr, *dw = nullptr, *w = nullptr;
+template <typename T> struct Args {
+    const T *b = nullptr, *r = nullptr, *dw = nullptr, *w = nullptr;
     const int32_t *prp = nullptr, *pci = nullptr;  // EP_FINAL: P by rows and the coarse block it multiplies
-    const float *pv = nullptr, *e = nullptr;
+    const T *pv = nullptr, *e = nullptr;
     double *part = nullptr;                        // DOT: column partials of b . y
     int NB = 0;                                    // their block rows
 };
 
-__device__ __forceinline__ void axpy4(float4 &y, float v, const float4 &x) {
-    y.x = fmaf(v, x.x, y.x);
-    y.y = fmaf(v, x.y, y.y);
-    y.z = fmaf(v, x.z, y.z);
-    y.w = fmaf(v, x.w, y.w);
+template <typename T, typename V> __device__ __forceinline__ void axpy4(V &y, T v, const V &x) {
+    y.x = fma(v, x.x, y.x);
+    y.y = fma(v, x.y, y.y);
+    y.z = fma(v, x.z, y.z);
+    y.w = fma(v, x.w, y.w);
 }
 
-template <int CH, int SPLIT, int EP, bool DOT>
+template <typename T, int CH, int SPLIT, int EP, bool DOT>
 __global__ void __launch_bounds__(kT, 2)
     k_ml_spmm(int64_t n, int64_t Rpad, int tile_rows, const int32_t *__restrict__ rowptr,
-              const int32_t *__restrict__ colidx, const float *__restrict__ vals, const float *__restrict__ x,
-              float *__restrict__ y, Args A) {
+              const int32_t *__restrict__ colidx, const T *__restrict__ vals, const T *__restrict__ x,
+              T *__restrict__ y, Args<T> A) {
+    using V = typename Four<T>::V;
     static_assert(SPLIT == 1 || (CH == 1 && !DOT), "split rows: one chunk, no partials");
     constexpr int ROWS = kGroups / SPLIT;  // rows of a block at a time
-    __shared__ float red[DOT ? kGroups : 1][DOT ? 32 * CH + 1 : 1];
+    __shared__ T red[DOT ? kGroups : 1][DOT ? 32 * CH + 1 : 1];
     const int l8 = threadIdx.x & 7, g = threadIdx.x >> 3, sub = SPLIT == 1 ? 0 : g % SPLIT;
     const int64_t t0 = (int64_t)blockIdx.y * 32 * CH + l8 * 4;
-    const float ws = (EP == EP_SCALE || EP == EP_FINAL) ? *A.w : 0.f;
-    float4 dot[CH];
+    const T ws = (EP == EP_SCALE || EP == EP_FINAL) ? *A.w : (T)0;
+    V dot[CH];
 #pragma unroll
-    for (int j = 0; j < CH; j++) dot[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < CH; j++) dot[j] = V{0, 0, 0, 0};
     const int64_t ntile = (n + tile_rows - 1) / tile_rows;
     for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x)
         for (int64_t row = tile * tile_rows + g / SPLIT, end = min(n, (tile + 1) * tile_rows); row < end; row += ROWS) {
-            float4 acc[CH];
+            V acc[CH];
 #pragma unroll
-            for (int j = 0; j < CH; j++) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int j = 0; j < CH; j++) acc[j] = V{0, 0, 0, 0};
             const int32_t s1 = rowptr[row + 1];
 #pragma unroll(CH == 1 ? 8 : 4)
             for (int32_t s = rowptr[row] + sub; s < s1; s += SPLIT) {
                 const int64_t col = colidx[s];
-                const float v = vals[s];
-                const float4 *xc = reinterpret_cast<const float4 *>(x + col * Rpad + t0);
+                const T v = vals[s];
+                const V *xc = reinterpret_cast<const V *>(x + col * Rpad + t0);
 #pragma unroll
-                for (int j = 0; j < CH; j++) axpy4(acc[j], v, __ldg(xc + 8 * j));
+                for (int j = 0; j < CH; j++) axpy4(acc[j], v, load4(xc + 8 * j));
             }
             if (SPLIT == 4) {
 #pragma unroll
@@ -232,43 +248,43 @@ __global__ void __launch_bounds__(kT, 2)
                 if (sub) continue;
             }
             const int64_t o = row * Rpad + t0;
-            float4 *yr = reinterpret_cast<float4 *>(y + o);
+            V *yr = reinterpret_cast<V *>(y + o);
             if (EP == EP_SCALE || EP == EP_FINAL) {
 #pragma unroll
-                for (int j = 0; j < CH; j++) acc[j] = make_float4(ws * acc[j].x, ws * acc[j].y, ws * acc[j].z, ws * acc[j].w);
+                for (int j = 0; j < CH; j++) acc[j] = V{ws * acc[j].x, ws * acc[j].y, ws * acc[j].z, ws * acc[j].w};
             }
             if (EP == EP_FINAL) {
                 for (int32_t p = A.prp[row], p1 = A.prp[row + 1]; p < p1; p++) {
-                    const float v = A.pv[p];
-                    const float4 *ec = reinterpret_cast<const float4 *>(A.e + (int64_t)A.pci[p] * Rpad + t0);
+                    const T v = A.pv[p];
+                    const V *ec = reinterpret_cast<const V *>(A.e + (int64_t)A.pci[p] * Rpad + t0);
 #pragma unroll
-                    for (int j = 0; j < CH; j++) axpy4(acc[j], v, __ldg(ec + 8 * j));
+                    for (int j = 0; j < CH; j++) axpy4(acc[j], v, load4(ec + 8 * j));
                 }
             }
             // every operand of the row is loaded before the first store
             constexpr bool B = EP == EP_RESID || EP == EP_POST || DOT;
-            float4 bv[B ? CH : 1], rv[EP == EP_POST || EP == EP_ACC ? CH : 1];
+            V bv[B ? CH : 1], rv[EP == EP_POST || EP == EP_ACC ? CH : 1];
 #pragma unroll
             for (int j = 0; j < CH; j++) {
-                if (B) bv[j] = __ldg(reinterpret_cast<const float4 *>(A.b + o) + 8 * j);
-                if (EP == EP_POST) rv[j] = __ldg(reinterpret_cast<const float4 *>(A.r + o) + 8 * j);
+                if (B) bv[j] = load4(reinterpret_cast<const V *>(A.b + o) + 8 * j);
+                if (EP == EP_POST) rv[j] = load4(reinterpret_cast<const V *>(A.r + o) + 8 * j);
                 if (EP == EP_ACC) rv[j] = yr[8 * j];
             }
-            const float dwi = EP == EP_POST ? A.dw[row] : 0.f;
+            const T dwi = EP == EP_POST ? A.dw[row] : (T)0;
 #pragma unroll
             for (int j = 0; j < CH; j++) {
-                float4 v = acc[j];
-                if (EP == EP_RESID) v = make_float4(bv[j].x - v.x, bv[j].y - v.y, bv[j].z - v.z, bv[j].w - v.w);
+                V v = acc[j];
+                if (EP == EP_RESID) v = V{bv[j].x - v.x, bv[j].y - v.y, bv[j].z - v.z, bv[j].w - v.w};
                 if (EP == EP_POST)
-                    v = make_float4(fmaf(dwi, bv[j].x + rv[j].x, v.x), fmaf(dwi, bv[j].y + rv[j].y, v.y),
-                                    fmaf(dwi, bv[j].z + rv[j].z, v.z), fmaf(dwi, bv[j].w + rv[j].w, v.w));
-                if (EP == EP_ACC) v = make_float4(rv[j].x + v.x, rv[j].y + v.y, rv[j].z + v.z, rv[j].w + v.w);
+                    v = V{fma(dwi, bv[j].x + rv[j].x, v.x), fma(dwi, bv[j].y + rv[j].y, v.y),
+                          fma(dwi, bv[j].z + rv[j].z, v.z), fma(dwi, bv[j].w + rv[j].w, v.w)};
+                if (EP == EP_ACC) v = V{rv[j].x + v.x, rv[j].y + v.y, rv[j].z + v.z, rv[j].w + v.w};
                 yr[8 * j] = v;
                 if (DOT) {
-                    dot[j].x = fmaf(bv[j].x, v.x, dot[j].x);
-                    dot[j].y = fmaf(bv[j].y, v.y, dot[j].y);
-                    dot[j].z = fmaf(bv[j].z, v.z, dot[j].z);
-                    dot[j].w = fmaf(bv[j].w, v.w, dot[j].w);
+                    dot[j].x = fma(bv[j].x, v.x, dot[j].x);
+                    dot[j].y = fma(bv[j].y, v.y, dot[j].y);
+                    dot[j].z = fma(bv[j].z, v.z, dot[j].z);
+                    dot[j].w = fma(bv[j].w, v.w, dot[j].w);
                 }
             }
         }
@@ -291,22 +307,23 @@ __global__ void __launch_bounds__(kT, 2)
 }
 
 // coarsest level: e = A^-1 b, one block per 8 rows and 32 columns with b's
-// columns in shared memory (8 KB at most)
-__global__ void __launch_bounds__(256) k_ml_dense(int n, int64_t Rpad, const float *__restrict__ inv,
-                                                  const float *__restrict__ b, float *__restrict__ e) {
-    __shared__ float bs[kMlCoarsest * 32];
+// columns in shared memory (16 KB at most)
+template <typename T>
+__global__ void __launch_bounds__(256) k_ml_dense(int n, int64_t Rpad, const T *__restrict__ inv,
+                                                  const T *__restrict__ b, T *__restrict__ e) {
+    __shared__ T bs[kMlCoarsest * 32];
     const int64_t c0 = (int64_t)blockIdx.y * 32;
     for (int t = threadIdx.x; t < n * 32; t += 256) bs[t] = b[(int64_t)(t >> 5) * Rpad + c0 + (t & 31)];
     __syncthreads();
     const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= n) return;
-    float s0 = 0.f, s1 = 0.f;
+    T s0 = 0, s1 = 0;
     int q = 0;
     for (; q + 1 < n; q += 2) {
-        s0 = fmaf(inv[row * n + q], bs[q * 32 + lane], s0);
-        s1 = fmaf(inv[row * n + q + 1], bs[(q + 1) * 32 + lane], s1);
+        s0 = fma(inv[row * n + q], bs[q * 32 + lane], s0);
+        s1 = fma(inv[row * n + q + 1], bs[(q + 1) * 32 + lane], s1);
     }
-    if (q < n) s0 = fmaf(inv[row * n + q], bs[q * 32 + lane], s0);
+    if (q < n) s0 = fma(inv[row * n + q], bs[q * 32 + lane], s0);
     e[(int64_t)row * Rpad + c0 + lane] = s0 + s1;
 }
 
@@ -342,14 +359,19 @@ __global__ void k_ml_damping(int NB, const double *__restrict__ part_xt, const d
     }
 }
 
+// T in a parameter that the others' types decide
+template <typename T> struct SameT { using type = T; };
+template <typename T> using Same = typename SameT<T>::type;
+
 // Rows per tile and columns per block: 128 rows and the widest column chunk
 // while that fills the SMs twice; shorter levels 32 rows (one per group) and 32
 // columns, and the shortest one row per warp.
-template <int EP, bool DOT>
-void spmm(cudaStream_t s, int64_t n, int64_t Rpad, const int32_t *rp, const int32_t *ci, const float *v,
-          const float *x, float *y, const Args &a) {
+template <int EP, bool DOT, typename T>
+void spmm(cudaStream_t s, int64_t n, int64_t Rpad, const int32_t *rp, const int32_t *ci, const T *v,
+          const Same<T> *x, T *y, const Args<Same<T>> &a) {
     const int64_t chunks = Rpad / 32;
     int ch = chunks % 4 == 0 ? 4 : chunks % 3 == 0 ? 3 : chunks % 2 == 0 ? 2 : 1;
+    if (sizeof(T) == 8) ch = chunks % 2 == 0 ? 2 : 1;  // registers; the FP64 pipe is the bound
     int tile = 128;
     bool split = false;
     if (ceil_div(n, tile) * (chunks / ch) < kFill) {
@@ -365,14 +387,22 @@ void spmm(cudaStream_t s, int64_t n, int64_t Rpad, const int32_t *rp, const int3
     const int64_t gx = DOT ? a.NB : std::min<int64_t>(ceil_div(n, tile), 4096);
     const dim3 g((unsigned)gx, (unsigned)(chunks / ch));
     if (split) {
-        if constexpr (!DOT) k_ml_spmm<1, 4, EP, false><<<g, kT, 0, s>>>(n, Rpad, tile, rp, ci, v, x, y, a);
+        if constexpr (!DOT) k_ml_spmm<T, 1, 4, EP, false><<<g, kT, 0, s>>>(n, Rpad, tile, rp, ci, v, x, y, a);
         return;
     }
+    if constexpr (sizeof(T) == 4) {
+        if (ch == 4) {
+            k_ml_spmm<T, 4, 1, EP, DOT><<<g, kT, 0, s>>>(n, Rpad, tile, rp, ci, v, x, y, a);
+            return;
+        }
+        if (ch == 3) {
+            k_ml_spmm<T, 3, 1, EP, DOT><<<g, kT, 0, s>>>(n, Rpad, tile, rp, ci, v, x, y, a);
+            return;
+        }
+    }
     switch (ch) {
-        case 4: k_ml_spmm<4, 1, EP, DOT><<<g, kT, 0, s>>>(n, Rpad, tile, rp, ci, v, x, y, a); break;
-        case 3: k_ml_spmm<3, 1, EP, DOT><<<g, kT, 0, s>>>(n, Rpad, tile, rp, ci, v, x, y, a); break;
-        case 2: k_ml_spmm<2, 1, EP, DOT><<<g, kT, 0, s>>>(n, Rpad, tile, rp, ci, v, x, y, a); break;
-        default: k_ml_spmm<1, 1, EP, DOT><<<g, kT, 0, s>>>(n, Rpad, tile, rp, ci, v, x, y, a); break;
+        case 2: k_ml_spmm<T, 2, 1, EP, DOT><<<g, kT, 0, s>>>(n, Rpad, tile, rp, ci, v, x, y, a); break;
+        default: k_ml_spmm<T, 1, 1, EP, DOT><<<g, kT, 0, s>>>(n, Rpad, tile, rp, ci, v, x, y, a); break;
     }
 }
 
@@ -425,17 +455,16 @@ void build(Context &c, cudaStream_t s) {
             l->PT_rp.upload(h.PT_rp, s);
             l->PT_ci.upload(h.PT_ci, s);
             l->PT_v.upload(h.PT_v, s);
+            l->PT64.upload(std::vector<double>(h.PT_v.begin(), h.PT_v.end()), s);
+            ERTGB_CUDA(cudaStreamSynchronize(s));  // the copy's source ends here
             l->AP_rp.upload(h.AP_rp, s);
             l->AP_ci.upload(h.AP_ci, s);
             l->AP.alloc((size_t)l->nnzAP);
-            l->Q.alloc((size_t)l->nnzAP);
-            l->dw.alloc((size_t)l->n);
         }
         M.levels.push_back(std::move(l));
     }
     const int64_t last = M.levels.back()->n;
     M.inv64.alloc((size_t)(last * last));
-    M.inv32.alloc((size_t)(last * last));
     M.bad.alloc(1);
     M.w.alloc(1);
     ERTGB_CUDA(cudaStreamSynchronize(s));  // host lists are freed on return
@@ -446,7 +475,35 @@ inline unsigned grid_rows(int64_t n, int per = kT) { return (unsigned)std::min<i
 
 }  // namespace
 
-static bool setup(Context &c, const double *fine, bool factor, int64_t Rpad, cudaStream_t s) {
+// largest eigenvalue of G^T G A from kPower power iterations on 32 columns
+static int factor_damping(Context &c, cudaStream_t s) {
+    MeshData &m = c.mesh;
+    Multilevel &M = m.ml;
+    const int NB = 152;
+    M.px.alloc((size_t)m.n * 32);
+    M.pt.alloc((size_t)m.n * 32);
+    M.pg.alloc((size_t)m.n * 32);
+    M.ppart.alloc((size_t)2 * NB * 32);
+    k_ml_start<<<grid_rows(m.n * 32), kT, 0, s>>>(m.n * 32, M.px.p);
+    for (int i = 0; i < kPower; i++) {
+        const bool end = i + 1 == kPower;
+        Args<float> a;
+        a.NB = NB;
+        a.b = M.px.p;
+        a.part = M.ppart.p;
+        if (end) spmm<EP_PLAIN, true>(s, m.n, 32, m.d_rowptr.p, m.d_colidx.p, c.d_S32.p, M.px.p, M.pt.p, a);
+        else spmm<EP_PLAIN, false>(s, m.n, 32, m.d_rowptr.p, m.d_colidx.p, c.d_S32.p, M.px.p, M.pt.p, a);
+        spmm<EP_PLAIN, false>(s, m.n, 32, m.d_Lrowptr.p, m.d_Lcolidx.p, c.d_G32.p, M.pt.p, M.pg.p, a);
+        a.b = M.pt.p;
+        a.part = M.ppart.p + NB * 32;
+        if (end) spmm<EP_PLAIN, true>(s, m.n, 32, m.d_Urowptr.p, m.d_Ucolidx.p, c.d_GT32.p, M.pg.p, M.px.p, a);
+        else spmm<EP_PLAIN, false>(s, m.n, 32, m.d_Urowptr.p, m.d_Ucolidx.p, c.d_GT32.p, M.pg.p, M.px.p, a);
+    }
+    k_ml_damping<<<1, 32, 0, s>>>(NB, M.ppart.p, M.ppart.p + NB * 32, M.w.p, M.bad.p);
+    return 3 * kPower + 2;
+}
+
+template <typename T> static bool setup(Context &c, const double *fine, bool factor, int64_t Rpad, cudaStream_t s) {
     MeshData &m = c.mesh;
     build(c, s);
     Multilevel &M = m.ml;
@@ -458,53 +515,36 @@ static bool setup(Context &c, const double *fine, bool factor, int64_t Rpad, cud
     for (size_t k = 0; k + 1 < L; k++) {
         MlLevel &l = *M.levels[k];
         MlLevel &d = *M.levels[k + 1];
+        MlValues<T> &v = l.values<T>();
         const int32_t *rp = k ? l.rp.p : m.d_rowptr.p, *ci = k ? l.ci.p : m.d_colidx.p;
         const double *val = k ? l.val.p : fine;
         const bool jac = k || !factor;
-        if (jac) l.AS.alloc((size_t)(k ? l.nnz : m.nnz));
-        k_ml_rows<<<grid_rows(32 * l.n), kT, 0, s>>>(l.n, rp, ci, val, l.P_rp.p, l.P_ci.p, l.P_v.p, l.AP_rp.p, l.AP_ci.p,
-                                                     jac ? 1 : 0, l.AP.p, l.dw.p, l.Q.p, M.bad.p);
-        if (jac) k_ml_scale<<<grid_rows(l.nnz), kT, 0, s>>>(l.nnz, ci, val, l.dw.p, l.AS.p);
+        if (jac) v.AS.alloc((size_t)l.nnz);
+        v.Q.alloc((size_t)l.nnzAP);
+        v.dw.alloc((size_t)l.n);
+        k_ml_rows<T><<<grid_rows(32 * l.n), kT, 0, s>>>(l.n, rp, ci, val, l.P_rp.p, l.P_ci.p, l.P_v.p, l.AP_rp.p, l.AP_ci.p,
+                                                     jac ? 1 : 0, l.AP.p, v.dw.p, v.Q.p, M.bad.p);
+        if (jac) k_ml_scale<T><<<grid_rows(l.nnz), kT, 0, s>>>(l.nnz, ci, val, v.dw.p, v.AS.p);
         k_ml_galerkin<<<grid_rows(32 * l.nc), kT, 0, s>>>(l.nc, l.PT_rp.p, l.PT_ci.p, l.PT_v.p, l.AP_rp.p, l.AP_ci.p,
                                                           l.AP.p, d.rp.p, d.ci.p, d.val.p);
         launches += 3;
         if (k) {
-            l.b.alloc((size_t)l.n * Rpad);
-            l.r.alloc((size_t)l.n * Rpad);
-            l.e.alloc((size_t)l.n * Rpad);
+            v.b.alloc((size_t)l.n * Rpad);
+            v.r.alloc((size_t)l.n * Rpad);
+            v.e.alloc((size_t)l.n * Rpad);
         }
     }
     MlLevel &z = *M.levels.back();
-    z.b.alloc((size_t)z.n * Rpad);
-    z.e.alloc((size_t)z.n * Rpad);
+    MlValues<T> &zv = z.values<T>();
+    zv.b.alloc((size_t)z.n * Rpad);
+    zv.e.alloc((size_t)z.n * Rpad);
+    zv.AS.alloc((size_t)(z.n * z.n));  // the inverse
     k_ml_densify<<<(unsigned)z.n, 128, 0, s>>>((int)z.n, z.rp.p, z.ci.p, z.val.p, M.inv64.p);
     dense_inverse(M.inv64.p, (int)z.n, M.bad.p, s);
-    k_ml_inverse32<<<grid_rows(z.n * z.n), kT, 0, s>>>((int)z.n, M.inv64.p, M.inv32.p);
+    k_ml_symmetric<T><<<grid_rows(z.n * z.n), kT, 0, s>>>((int)z.n, M.inv64.p, zv.AS.p);
     launches += 3;
-    if (factor) {
-        // largest eigenvalue of G^T G A from kPower power iterations on 32 columns
-        const int NB = 152;
-        M.px.alloc((size_t)m.n * 32);
-        M.pt.alloc((size_t)m.n * 32);
-        M.pg.alloc((size_t)m.n * 32);
-        M.ppart.alloc((size_t)2 * NB * 32);
-        k_ml_start<<<grid_rows(m.n * 32), kT, 0, s>>>(m.n * 32, M.px.p);
-        for (int i = 0; i < kPower; i++) {
-            const bool end = i + 1 == kPower;
-            Args a;
-            a.NB = NB;
-            a.b = M.px.p;
-            a.part = M.ppart.p;
-            if (end) spmm<EP_PLAIN, true>(s, m.n, 32, m.d_rowptr.p, m.d_colidx.p, c.d_S32.p, M.px.p, M.pt.p, a);
-            else spmm<EP_PLAIN, false>(s, m.n, 32, m.d_rowptr.p, m.d_colidx.p, c.d_S32.p, M.px.p, M.pt.p, a);
-            spmm<EP_PLAIN, false>(s, m.n, 32, m.d_Lrowptr.p, m.d_Lcolidx.p, c.d_G32.p, M.pt.p, M.pg.p, a);
-            a.b = M.pt.p;
-            a.part = M.ppart.p + NB * 32;
-            if (end) spmm<EP_PLAIN, true>(s, m.n, 32, m.d_Urowptr.p, m.d_Ucolidx.p, c.d_GT32.p, M.pg.p, M.px.p, a);
-            else spmm<EP_PLAIN, false>(s, m.n, 32, m.d_Urowptr.p, m.d_Ucolidx.p, c.d_GT32.p, M.pg.p, M.px.p, a);
-        }
-        k_ml_damping<<<1, 32, 0, s>>>(NB, M.ppart.p, M.ppart.p + NB * 32, M.w.p, M.bad.p);
-        launches += 3 * kPower + 2;
+    if constexpr (sizeof(T) == 4) {
+        if (factor) launches += factor_damping(c, s);
     }
     ERTGB_CUDA(cudaGetLastError());
     int32_t bad = 0;
@@ -514,16 +554,18 @@ static bool setup(Context &c, const double *fine, bool factor, int64_t Rpad, cud
     return bad == 0;
 }
 
-bool ml_setup(Context &c, const double *val, bool factor, int64_t cols, cudaStream_t s) {
+// 3-D (one wavenumber k = 0): the 2.5-D path has its direct solve.  One response
+// without -> with coarse levels: 1350 nodes, 12 electrodes 5.2 -> 2.3 ms
+// (Jacobi), 4.0 -> 2.2 (FSAI); 4224 nodes, 48 electrodes 11.9 -> 3.2, 11.6 ->
+// 3.5; nothing smaller than kMlMinRows was measured.  CEM and bypass matrices
+// keep the single level.
+template <typename T>
+static bool guarded_setup(Context &c, const double *val, bool factor, int64_t cols, cudaStream_t s) {
     const MeshData &m = c.mesh;
-    // 3-D (one wavenumber k = 0): the 2.5-D path has its direct solve.  One response
-    // without -> with coarse levels: 1350 nodes, 12 electrodes 5.2 -> 2.3 ms
-    // (Jacobi), 4.0 -> 2.2 (FSAI); 4224 nodes, 48 electrodes 11.9 -> 3.2, 11.6 ->
-    // 3.5; nothing smaller than kMlMinRows was measured
-    if (m.dim != 3 || c.nK != 1 || c.k[0] != 0.0 || m.n < kMlMinRows) return false;
-    if (!m.ext_rows.empty() || m.n_ext > 0) return false;  // CEM and bypass matrices keep the single level
+    if (!c.coarse_levels || m.dim != 3 || c.nK != 1 || c.k[0] != 0.0 || m.n < kMlMinRows) return false;
+    if (!m.ext_rows.empty() || m.n_ext > 0) return false;
     try {
-        return setup(c, val, factor, cols, s);
+        return setup<T>(c, val, factor, cols, s);
     } catch (Error &e) {
         if (e.code != ERTGB_OOM) throw;
         // the coarse levels do not fit beside the rest: the single-level form does without
@@ -538,64 +580,90 @@ bool ml_setup(Context &c, const double *val, bool factor, int64_t cols, cudaStre
     }
 }
 
-void ml_cycle(Context &c, const MlBlock &v, int NB, double *pz, cudaStream_t s) {
+bool ml_setup(Context &c, const double *val, bool factor, int64_t cols, cudaStream_t s) {
+    return guarded_setup<float>(c, val, factor, cols, s);
+}
+
+bool ml_setup64(Context &c, const double *val, int64_t cols, cudaStream_t s) {
+    return guarded_setup<double>(c, val, false, cols, s);
+}
+
+template <typename T>
+static void cycle(Context &c, const MlBlock<T> &v, int NB, double *pz, cudaStream_t s) {
     MeshData &m = c.mesh;
     Multilevel &M = m.ml;
     const int64_t n = m.n, R = v.cols;
     const size_t L = M.levels.size();
     MlLevel &f = *M.levels[0];
-    const float *b = v.b;
-    float *z = v.z, *r = v.r, *t = v.t;
-    Args a;
-    if (M.factor) {
-        a.w = M.w.p;
-        spmm<EP_PLAIN, false>(s, n, R, m.d_Lrowptr.p, m.d_Lcolidx.p, c.d_G32.p, b, t, a);
-        spmm<EP_SCALE, false>(s, n, R, m.d_Urowptr.p, m.d_Ucolidx.p, c.d_GT32.p, t, z, a);
-        a.b = b;
-        spmm<EP_RESID, false>(s, n, R, m.d_rowptr.p, m.d_colidx.p, c.d_S32.p, z, r, a);
-    } else {
-        a.b = b;
-        spmm<EP_RESID, false>(s, n, R, m.d_rowptr.p, m.d_colidx.p, f.AS.p, b, r, a);
+    MlValues<T> &fv = f.values<T>();
+    const T *b = v.b;
+    T *z = v.z, *r = v.r;
+    Args<T> a;
+    a.b = b;
+    bool factor = false;
+    if constexpr (sizeof(T) == 4) {
+        factor = M.factor;
+        if (factor) {
+            a.w = M.w.p;
+            spmm<EP_PLAIN, false>(s, n, R, m.d_Lrowptr.p, m.d_Lcolidx.p, c.d_G32.p, b, v.t, a);
+            spmm<EP_SCALE, false>(s, n, R, m.d_Urowptr.p, m.d_Ucolidx.p, c.d_GT32.p, v.t, z, a);
+            spmm<EP_RESID, false>(s, n, R, m.d_rowptr.p, m.d_colidx.p, c.d_S32.p, z, r, a);
+        }
     }
-    spmm<EP_PLAIN, false>(s, f.nc, R, f.PT_rp.p, f.PT_ci.p, f.PT_v.p, r, M.levels[1]->b.p, Args{});
+    if (!factor) spmm<EP_RESID, false>(s, n, R, m.d_rowptr.p, m.d_colidx.p, fv.AS.p, b, r, a);
+    auto restrict_to = [&](MlLevel &l, const T *from, T *to) {
+        if constexpr (sizeof(T) == 4) spmm<EP_PLAIN, false>(s, l.nc, R, l.PT_rp.p, l.PT_ci.p, l.PT_v.p, from, to, Args<T>{});
+        else spmm<EP_PLAIN, false>(s, l.nc, R, l.PT_rp.p, l.PT_ci.p, l.PT64.p, from, to, Args<T>{});
+    };
+    restrict_to(f, r, M.levels[1]->values<T>().b.p);
     for (size_t k = 1; k + 1 < L; k++) {
         MlLevel &l = *M.levels[k];
-        Args q;
-        q.b = l.b.p;
-        spmm<EP_RESID, false>(s, l.n, R, l.rp.p, l.ci.p, l.AS.p, l.b.p, l.r.p, q);
-        spmm<EP_PLAIN, false>(s, l.nc, R, l.PT_rp.p, l.PT_ci.p, l.PT_v.p, l.r.p, M.levels[k + 1]->b.p, Args{});
+        MlValues<T> &lv = l.values<T>();
+        Args<T> q;
+        q.b = lv.b.p;
+        spmm<EP_RESID, false>(s, l.n, R, l.rp.p, l.ci.p, lv.AS.p, lv.b.p, lv.r.p, q);
+        restrict_to(l, lv.r.p, M.levels[k + 1]->values<T>().b.p);
     }
     MlLevel &d = *M.levels[L - 1];
-    k_ml_dense<<<dim3((unsigned)ceil_div(d.n, 8), (unsigned)(R / 32)), 256, 0, s>>>((int)d.n, R, M.inv32.p, d.b.p,
-                                                                                    d.e.p);
+    MlValues<T> &dv = d.values<T>();
+    k_ml_dense<T><<<dim3((unsigned)ceil_div(d.n, 8), (unsigned)(R / 32)), 256, 0, s>>>((int)d.n, R, dv.AS.p, dv.b.p,
+                                                                                       dv.e.p);
     for (size_t k = L - 2; k >= 1; k--) {
         MlLevel &l = *M.levels[k];
-        Args q;
-        q.b = l.b.p;
-        q.r = l.r.p;
-        q.dw = l.dw.p;
-        spmm<EP_POST, false>(s, l.n, R, l.AP_rp.p, l.AP_ci.p, l.Q.p, M.levels[k + 1]->e.p, l.e.p, q);
+        MlValues<T> &lv = l.values<T>();
+        Args<T> q;
+        q.b = lv.b.p;
+        q.r = lv.r.p;
+        q.dw = lv.dw.p;
+        spmm<EP_POST, false>(s, l.n, R, l.AP_rp.p, l.AP_ci.p, lv.Q.p, M.levels[k + 1]->values<T>().e.p,
+                             lv.e.p, q);
     }
-    const float *e = M.levels[1]->e.p;
-    a.b = b;
+    const T *e = M.levels[1]->values<T>().e.p;
     a.part = pz;
     a.NB = NB;
-    if (M.factor) {
-        spmm<EP_ACC, false>(s, n, R, f.AP_rp.p, f.AP_ci.p, f.Q.p, e, r, Args{});
-        spmm<EP_ACC, false>(s, n, R, m.d_Lrowptr.p, m.d_Lcolidx.p, c.d_G32.p, r, t, Args{});
-        a.prp = f.P_rp.p;
-        a.pci = f.P_ci.p;
-        a.pv = f.P_v.p;
-        a.e = e;
-        spmm<EP_FINAL, true>(s, n, R, m.d_Urowptr.p, m.d_Ucolidx.p, c.d_GT32.p, t, z, a);
-    } else {
+    if constexpr (sizeof(T) == 4) {
+        if (factor) {
+            spmm<EP_ACC, false>(s, n, R, f.AP_rp.p, f.AP_ci.p, fv.Q.p, e, r, Args<T>{});
+            spmm<EP_ACC, false>(s, n, R, m.d_Lrowptr.p, m.d_Lcolidx.p, c.d_G32.p, r, v.t, Args<T>{});
+            a.prp = f.P_rp.p;
+            a.pci = f.P_ci.p;
+            a.pv = f.P_v.p;
+            a.e = e;
+            spmm<EP_FINAL, true>(s, n, R, m.d_Urowptr.p, m.d_Ucolidx.p, c.d_GT32.p, v.t, z, a);
+        }
+    }
+    if (!factor) {
         a.r = r;
-        a.dw = f.dw.p;
-        if (pz) spmm<EP_POST, true>(s, n, R, f.AP_rp.p, f.AP_ci.p, f.Q.p, e, z, a);
-        else spmm<EP_POST, false>(s, n, R, f.AP_rp.p, f.AP_ci.p, f.Q.p, e, z, a);
+        a.dw = fv.dw.p;
+        if (pz) spmm<EP_POST, true>(s, n, R, f.AP_rp.p, f.AP_ci.p, fv.Q.p, e, z, a);
+        else spmm<EP_POST, false>(s, n, R, f.AP_rp.p, f.AP_ci.p, fv.Q.p, e, z, a);
     }
     ERTGB_CUDA(cudaGetLastError());
 }
+
+void ml_cycle(Context &c, const MlBlock<float> &v, int NB, double *pz, cudaStream_t s) { cycle(c, v, NB, pz, s); }
+
+void ml_cycle64(Context &c, const MlBlock<double> &v, int NB, double *pz, cudaStream_t s) { cycle(c, v, NB, pz, s); }
 
 int ml_launches(const Context &c) {
     const Multilevel &M = c.mesh.ml;

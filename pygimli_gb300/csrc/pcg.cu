@@ -30,6 +30,7 @@ namespace {
 
 constexpr int kRowsPerBlock = 8;  // warps per block in spmm, rows per block in vector kernels
 constexpr int kGraphIters = 16;
+constexpr int kMlIters = 4;  // iterations per graph (and host check) with coarse levels
 constexpr int kPartRows = 608;  // block partial rows of every column reduction (4 x 152 SMs)
 
 
@@ -387,8 +388,21 @@ int pcg_solve(Context &c, cudaStream_t s, const int32_t *mask) {
     ERTGB_CUDA(cudaMemsetAsync(nactive, 0, sizeof(int32_t), s));
     // IC(0) (plain FP64 solve only; the FP64 finish of the mixed solver keeps Jacobi)
     const bool ic0 = c.precond == ERTGB_PRECOND_IC0 && !mask;
-    const double *dv = ic0 ? nullptr : c.d_dinv.p;
+    // coarse levels around Jacobi (3-D); the FP64 finish of the mixed solver's
+    // stalled columns keeps the single level
+    const bool ml = c.precond == ERTGB_PRECOND_JACOBI && c.precision == ERTGB_PRECISION_FP64 && !mask &&
+                    ml_setup64(c, c.d_S.p, Rpad, s);
+    const bool zform = ic0 || ml;  // z = M^-1 r is a product of its own
+    const double *dv = zform ? nullptr : c.d_dinv.p;
     const double *zg = nullptr;
+    // z = M^-1 r with the partials of r . z (q is free between the residual's update and the operator)
+    auto ml_apply = [&] { ml_cycle64(c, MlBlock<double>{Rpad, c.d_r.p, c.d_z.p, c.d_q.p, nullptr}, NB, part_a, s); };
+    if (ml) {
+        c.d_z.alloc((size_t)n * Rpad);
+        ml_apply();
+        zg = c.d_z.p;
+        c.stats.launches_response += ml_launches(c);
+    }
     if (ic0) {
         ic0_setup(c, s);
         c.d_z.alloc((size_t)n * Rpad);
@@ -405,7 +419,10 @@ int pcg_solve(Context &c, cudaStream_t s, const int32_t *mask) {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     ERTGB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    for (int it = 0; it < kGraphIters; it++) {
+    const int graph_iters = ml ? kMlIters : kGraphIters;
+    // with coarse levels a column goes one digit below the tolerance, as in the mixed solver (k_m_finish_ml)
+    const double stop2 = ml ? 0.01 * rtol2 : rtol2;
+    for (int it = 0; it < graph_iters; it++) {
         launch_spmm(ch, sg, s, n, m.nnz, c.nE, c.nK, Rpad, m.d_rowptr.p, m.d_colidx.p, c.d_S.p, c.d_p.p, c.d_q.p,
                     part_c, active);
         k_finish_alpha_w<<<fwg, 32 * kFinWarps, 0, s>>>(Rpad, NB, part_c, c.d_col.p, active, nactive);
@@ -415,7 +432,8 @@ int pcg_solve(Context &c, cudaStream_t s, const int32_t *mask) {
             ic0_apply(c, c.d_r.p, c.d_z.p, s);
             k_dot_rz<<<vg, vb, 0, s>>>(n, Rpad, active, c.d_r.p, c.d_z.p, part_a);
         }
-        k_finish_beta_w<<<fwg, 32 * kFinWarps, 0, s>>>(Rpad, NB, rtol2, part_a, part_b, c.d_col.p, active, iters,
+        if (ml) ml_apply();
+        k_finish_beta_w<<<fwg, 32 * kFinWarps, 0, s>>>(Rpad, NB, stop2, part_a, part_b, c.d_col.p, active, iters,
                                                        nactive);
         k_update_p<<<vg, vb, 0, s>>>(n, c.nE, R, Rpad, dv, c.d_col.p, active, c.d_r.p, c.d_p.p, zg);
     }
@@ -439,8 +457,8 @@ int pcg_solve(Context &c, cudaStream_t s, const int32_t *mask) {
                 break;
             }
             ERTGB_CUDA(cudaGraphLaunch(exec, s));
-            iterations += kGraphIters;
-            c.stats.launches_response += (5 + (ic0 ? ic0_launches(c) + 1 : 0)) * kGraphIters;
+            iterations += graph_iters;
+            c.stats.launches_response += (5 + (ic0 ? ic0_launches(c) + 1 : ml ? ml_launches(c) : 0)) * graph_iters;
             ERTGB_CUDA(cudaMemcpyAsync(&h_active, nactive, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
             ERTGB_CUDA(cudaStreamSynchronize(s));
         }

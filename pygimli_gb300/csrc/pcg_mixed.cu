@@ -667,7 +667,7 @@ int pcg_solve_mixed(Context &c, cudaStream_t s) {
     auto apply_fsai = [&](double *pz) {
         if (ml) {
             // q is free between the residual's update and the operator
-            ml_cycle(c, MlBlock{Rpad, c.d_r32.p, c.d_z32.p, c.d_q32.p, c.d_t32.p}, NB, pz, s);
+            ml_cycle(c, MlBlock<float>{Rpad, c.d_r32.p, c.d_z32.p, c.d_q32.p, c.d_t32.p}, NB, pz, s);
             return;
         }
         dispatch_ch<GenL>(ch, dim3((unsigned)NB, (unsigned)nchunk), s, n, nL, c.nE, c.nK, Rpad, m.d_Lrowptr.p,

@@ -271,6 +271,12 @@ class ERTModelling:
         self._precond = codes[precond]
         self._check(self._lib.ertgb_set_solver(self._ctx, self._rtol, self._maxIter, self._precond))
 
+    def setCoarseLevels(self, on=True):
+        """Coarse levels of the iterative solvers on 3-D meshes (default on):
+        the preconditioner becomes the fine-level smoother of a multilevel
+        cycle.  ``False``: the preconditioner alone, the plain PCG."""
+        self._check(self._lib.ertgb_set_coarse_levels(self._ctx, 1 if on else 0))
+
     def createRefinedFwdMesh(self, mesh):
         """Forward mesh of a parameter mesh: H2 refinement, then P2, as
         enabled by ``_refineH2`` / ``_refineP2``

@@ -1,5 +1,5 @@
-"""Coarse levels of the mixed-precision solver (3-D meshes of at least 1024
-nodes) against the plain FP64 PCG at rtol 1e-12: every fine-level smoother,
+"""Coarse levels of the mixed-precision and the FP64 solver (3-D meshes of at least
+1024 nodes) against the plain FP64 PCG at rtol 1e-12: every fine-level smoother,
 ground and boundary condition that the solver takes, repeated passes on one
 operator, changed models and fixed rows.
 
@@ -56,7 +56,15 @@ def operator(mesh, data, **kw):
     return f
 
 
+def plain(mesh, data, **kw):
+    f = operator(mesh, data, rtol=1e-12, **kw)
+    f.setCoarseLevels(False)
+    return f
+
+
 def mixed(mesh, data, precond, **kw):
+    if precond == "fp64":
+        return operator(mesh, data, **kw)
     if precond == "learned":
         import pygimli_gb300
         kw["weights"] = os.path.join(os.path.dirname(pygimli_gb300.__file__), "weights", "box_3d.npz")
@@ -75,22 +83,22 @@ def agree(fast, exact, rho):
 
 
 @pytest.mark.parametrize("kind", ["random", "contrast", "homogeneous"])
-@pytest.mark.parametrize("precond", ["jacobi", "fsai", "learned"])
+@pytest.mark.parametrize("precond", ["jacobi", "fsai", "learned", "fp64"])
 def test_smoothers(torch, precond, kind):
     mesh, data = box()
     assert mesh.nodeCount() >= 8192
-    fast, exact = mixed(mesh, data, precond), operator(mesh, data, rtol=1e-12)
+    fast, exact = mixed(mesh, data, precond), plain(mesh, data)
     for seed in (1, 2):  # the levels' patterns are kept, their values are not
         agree(fast, exact, ground(mesh, kind, seed))
 
 
-@pytest.mark.parametrize("precond", ["jacobi", "fsai"])
+@pytest.mark.parametrize("precond", ["jacobi", "fsai", "fp64"])
 def test_quadratic_and_tight(torch, precond):
     """P2 matrices (positive couplings, long rows) and rtol 1e-12."""
     mesh, data = box(nx=4, ny=3, h=4.0)
     mesh = mesh.createP2()
     assert mesh.nodeCount() >= 8192
-    agree(mixed(mesh, data, precond, rtol=1e-12), operator(mesh, data, rtol=1e-12), ground(mesh, "random"))
+    agree(mixed(mesh, data, precond, rtol=1e-12), plain(mesh, data), ground(mesh, "random"))
 
 
 def with_markers(mesh, bm, nm=None):
@@ -100,7 +108,8 @@ def with_markers(mesh, bm, nm=None):
 
 @pytest.mark.parametrize("sr", [True, False])
 @pytest.mark.parametrize("where", ["sides", "all"])
-def test_dirichlet(torch, sr, where):
+@pytest.mark.parametrize("precond", ["fsai", "fp64"])
+def test_dirichlet(torch, sr, where, precond):
     """Rows without couplings (homogeneous Dirichlet nodes) stay out of the
     coarse levels."""
     mesh, data = box()
@@ -108,7 +117,7 @@ def test_dirichlet(torch, sr, where):
     c = mesh.nodes[mesh.boundaries].mean(axis=1)
     bm[(bm == -2) & ((c[:, 2] > c[:, 2].min() + 1e-6) | (where == "all"))] = -3
     m = with_markers(mesh, bm)
-    agree(mixed(m, data, "fsai", sr=sr), operator(m, data, rtol=1e-12, sr=sr), ground(m, "random"))
+    agree(mixed(m, data, precond, sr=sr), plain(m, data, sr=sr), ground(m, "random"))
 
 
 def test_closed_domain(torch):
@@ -128,7 +137,7 @@ def test_closed_domain(torch):
             fast = mixed(m, data, "fsai", sr=False)
         else:
             fast.setMesh(m, ignoreRegionManager=True)
-        agree(fast, operator(m, data, rtol=1e-12, sr=False), ground(m, "random"))
+        agree(fast, plain(m, data, sr=False), ground(m, "random"))
 
 
 
@@ -139,7 +148,7 @@ def test_complex(torch, phase):
     sources leaves padded columns."""
     mesh, data = box()
     rng = np.random.default_rng(3)
-    fast, exact = operator(mesh, data, precision="mixed"), operator(mesh, data, rtol=1e-12)
+    fast, exact = operator(mesh, data, precision="mixed"), plain(mesh, data)
     fast.setComplex(True)
     exact.setComplex(True)
     for seed in (1, 2):
