@@ -191,7 +191,7 @@ struct JacTiles {
 // infinity), and the records of each chunk sorted by current dipole (datum,
 // ia | im << 16, geometric factor).
 struct JacStiff {
-    bool ok = false;
+    bool ok = false, node_build = false;
     int nchunks = 0, RS = 0;  // chunks, staged row length (columns)
     int64_t ntiles = 0;
     size_t tab_bytes = 0, stage_bytes = 0, smem = 0;

@@ -238,11 +238,23 @@ __global__ void k_jac_scales(int64_t D, int64_t P, const double *__restrict__ kf
 // memory with the next batch loaded ahead; 16 lanes per record, each lane two
 // adjacent parameters: nv-1 conflict-free 8-byte table loads, 2(nv-1) FMAs and
 // one 8-byte J store (two 4-byte stores when P is odd).
+//
+// FP32 J of P1 cells with at most 32 distinct nodes per tile (FB): the potential
+// rows are staged electrode by electrode (kNS nodes each), and a warp builds a
+// table row with its lanes first as nodes, then as slots: the dipole's
+// difference u_a - u_b at every node as an error-free FP32 pair (Knuth's
+// two-sum on the hi parts, its error added to the lo difference), handed to the
+// slots by shuffles, and K_c from registers.  The general build reads every
+// node of every slot for both electrodes, 8 strided 8-byte loads and 9 of K_c
+// against 2 contiguous ones and 8 shuffles; with 2940 distinct dipoles
+// (box_3d_large, ten chunks per tile) it was five sixths of the kernel: 21.3 ->
+// 14.8 ms, box_3d (1200 dipoles) 3.30 -> 2.97 ms, 23k nodes 1.16 -> 0.92 ms.
 // ---------------------------------------------------------------------------
 
 constexpr int kSJT = 1024;  // threads of the stiffness kernel (one block per SM)
 constexpr int kSTW = 32;    // parameters per tile
 constexpr int kNREC = 16;   // data records staged per warp batch
+constexpr int kNS = 33;     // FB: staged nodes per electrode (odd: rows of electrodes start 2 banks apart)
 
 // chunk descriptor: data range of the sorted records, dipoles and their offsets
 struct StiffChunk {
@@ -273,6 +285,11 @@ template <> __device__ __forceinline__ double record_scale<double>(int4 m) {
     return __hiloint2double(m.w, m.z);
 }
 
+// asynchronous 8-byte global -> shared copy (both addresses 8-byte aligned)
+__device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s), "l"(gmem) : "memory");
+}
 // asynchronous 16-byte global -> shared copy (both addresses 16-byte aligned)
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -286,7 +303,7 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // VEC: 4 = four adjacent parameters per lane and 16-byte stores (FP32 J with
 // a row length and base aligned to four), 2 = two per lane and paired
 // stores, 1 = two per lane, element stores
-template <int NV, typename OT, int VEC>
+template <int NV, typename OT, int VEC, bool FB>
 __global__ void __launch_bounds__(kSJT, 1)
     k_jac_stiff(int64_t ntiles, int64_t P, const int32_t *__restrict__ pc, const double *__restrict__ K,
                 const typename StageOf<OT>::type *__restrict__ pot, int64_t Rpad, int nE, int RS,
@@ -304,6 +321,7 @@ __global__ void __launch_bounds__(kSJT, 1)
     constexpr int LPR = TW / PPL;      // lanes per record
     constexpr int RPW = 32 / LPR;      // records per warp step
     static_assert(VEC != 4 || sizeof(OT) == 4, "16-byte stores of four FP32 values");
+    static_assert(!FB || (sizeof(OT) == 4 && NV <= 4), "the node-wise build is for FP32 J of P1 cells");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // [TA | TM tables: row = NM1 x TW values, slot fastest][staged rows Us]
     // [Ks: TW x NM1^2][sps: TW][lid: TW x NV bytes][records: NW x kNREC x (scale, datum, dipoles)]
@@ -342,7 +360,13 @@ __global__ void __launch_bounds__(kSJT, 1)
         __syncthreads();  // the previous tile is done with every shared buffer
         // the tile's node rows: columns [0, nE2) by 16-byte copies, an odd last column by a
         // plain load, column nE (the electrode at infinity) zero
-        {
+        if constexpr (FB) {
+            for (int q = threadIdx.x; q < nn * nE; q += kSJT) {
+                const int i = q / nE, e = q - i * nE;
+                cp_async8(Us + e * kNS + i, pot + (int64_t)tnodes[n0 + i] * Rpad + e);
+            }
+            for (int i = threadIdx.x; i < nn; i += kSJT) Us[nE * kNS + i] = ST{};
+        } else {
             const int per = nE2 / 2;
             for (int q = threadIdx.x; q < nn * per; q += kSJT) {
                 const int i = q / per, c2 = 2 * (q - i * per);
@@ -369,33 +393,88 @@ __global__ void __launch_bounds__(kSJT, 1)
             OT *TA = tabs;
             OT *TM = tabs + (size_t)cd.nA * NM1 * TW;
             __syncthreads();  // staged rows, lid, sps, Ks visible; the previous chunk's pair phase is done
-            // TA rows (w_0 / model^2 * K_c g_ab) and TM rows (g_mn) of the chunk's dipoles:
-            // thread = (dipole, slot), slot fastest
-            for (int q = threadIdx.x; q < (cd.nA + cd.nM) * TW; q += kSJT) {
-                const int g = q % TW;
-                int dp = q / TW;
-                const bool isA = dp < cd.nA;
-                if (!isA) dp -= cd.nA;
-                const int32_t *dd = isA ? dac : dmc;
-                OT gv[NM1], out[NM1];
-                const bool ok = shifted(g, dd[2 * dp], dd[2 * dp + 1], gv);
-                if (isA) {
-                    const OT *Kg = Ks + (size_t)g * NM1 * NM1;
-                    const OT f = sps[g];
+            if constexpr (FB) {
+                // lane = node, then slot: this slot's local nodes (0xff: empty), K_c and scale
+                int ln[NV];
 #pragma unroll
-                    for (int i = 0; i < NM1; i++) {
-                        OT sacc = 0;
+                for (int j = 0; j < NV; j++) ln[j] = lid[lane * NV + j];
+                const bool full = ln[0] != 0xff;
+                OT Kr[NM1 * NM1];
 #pragma unroll
-                        for (int j = 0; j < NM1; j++) sacc = fma(Kg[i * NM1 + j], gv[j], sacc);
-                        out[i] = ok ? sacc * f : (OT)0;
+                for (int i = 0; i < NM1 * NM1; i++) Kr[i] = Ks[lane * NM1 * NM1 + i] * sps[lane];
+                const int ndip = cd.nA + cd.nM;
+                for (int first = warp; first < ndip; first += 32 * NW) {
+                    // lane k holds the electrodes of the warp's k-th dipole
+                    int da = nE, db = nE;
+                    const int mine = first + NW * lane;
+                    if (mine < ndip) {
+                        const int32_t *dd = mine < cd.nA ? dac + 2 * mine : dmc + 2 * (mine - cd.nA);
+                        da = dd[0];
+                        db = dd[1];
                     }
-                } else {
+                    for (int k = 0; k < 32; k++) {
+                        const int dp = first + NW * k;
+                        if (dp >= ndip) break;  // warp-uniform
+                        const int a = __shfl_sync(0xffffffffu, da, k), b = __shfl_sync(0xffffffffu, db, k);
+                        float2 ua = make_float2(0.f, 0.f), ub = ua;
+                        if (lane < nn) {
+                            ua = Us[a * kNS + lane];
+                            ub = Us[b * kNS + lane];
+                        }
+                        const float dh = ua.x - ub.x, t = dh - ua.x;
+                        const float dl = ((ua.x - (dh - t)) + (-ub.x - t)) + (ua.y - ub.y);
+                        const float h0 = __shfl_sync(0xffffffffu, dh, ln[0]), l0 = __shfl_sync(0xffffffffu, dl, ln[0]);
+                        OT gv[NM1];
 #pragma unroll
-                    for (int i = 0; i < NM1; i++) out[i] = ok ? gv[i] : (OT)0;
+                        for (int j = 0; j < NM1; j++) {
+                            const float h = __shfl_sync(0xffffffffu, dh, ln[j + 1]);
+                            const float l = __shfl_sync(0xffffffffu, dl, ln[j + 1]);
+                            gv[j] = full ? (h - h0) + (l - l0) : (OT)0;
+                        }
+                        OT *dst = tabs + (size_t)dp * NM1 * TW + lane;
+                        if (dp < cd.nA) {
+#pragma unroll
+                            for (int i = 0; i < NM1; i++) {
+                                OT sacc = 0;
+#pragma unroll
+                                for (int j = 0; j < NM1; j++) sacc = fma(Kr[i * NM1 + j], gv[j], sacc);
+                                dst[i * TW] = sacc;
+                            }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < NM1; i++) dst[i * TW] = gv[i];
+                        }
+                    }
                 }
-                OT *dst = (isA ? TA : TM) + (size_t)dp * NM1 * TW + g;
+            } else {
+                // TA rows (w_0 / model^2 * K_c g_ab) and TM rows (g_mn) of the chunk's dipoles:
+                // thread = (dipole, slot), slot fastest
+                for (int q = threadIdx.x; q < (cd.nA + cd.nM) * TW; q += kSJT) {
+                    const int g = q % TW;
+                    int dp = q / TW;
+                    const bool isA = dp < cd.nA;
+                    if (!isA) dp -= cd.nA;
+                    const int32_t *dd = isA ? dac : dmc;
+                    OT gv[NM1], out[NM1];
+                    const bool ok = shifted(g, dd[2 * dp], dd[2 * dp + 1], gv);
+                    if (isA) {
+                        const OT *Kg = Ks + (size_t)g * NM1 * NM1;
+                        const OT f = sps[g];
 #pragma unroll
-                for (int i = 0; i < NM1; i++) dst[i * TW] = out[i];
+                        for (int i = 0; i < NM1; i++) {
+                            OT sacc = 0;
+#pragma unroll
+                            for (int j = 0; j < NM1; j++) sacc = fma(Kg[i * NM1 + j], gv[j], sacc);
+                            out[i] = ok ? sacc * f : (OT)0;
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < NM1; i++) out[i] = ok ? gv[i] : (OT)0;
+                    }
+                    OT *dst = (isA ? TA : TM) + (size_t)dp * NM1 * TW + g;
+#pragma unroll
+                    for (int i = 0; i < NM1; i++) dst[i * TW] = out[i];
+                }
             }
             __syncthreads();
             // pair phase: warp w streams a balanced range of the chunk's records (sorted by
@@ -538,7 +617,8 @@ void launch_stiff(Context &c, bool scaled, const CT *sp, CT *J, int dtype, cudaS
     ERTGB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.device));
     const CT w0 = (CT)c.w[0];
     auto go = [&](auto kern) {
-        ERTGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.smem));
+        // always the same limit: contexts may launch from several host threads
+        ERTGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStiffSmem));
         const int64_t grid = std::min<int64_t>(S.ntiles, (int64_t)nsm);
         kern<<<(unsigned)grid, kSJT, S.smem, s>>>(
             S.ntiles, m.P, S.d_pc.p, m.d_K.p, pot, c.Rpad, c.nE, S.RS, S.d_nptr.p, S.d_tnodes.p, S.d_lidx.p,
@@ -552,14 +632,22 @@ void launch_stiff(Context &c, bool scaled, const CT *sp, CT *J, int dtype, cudaS
     const bool v4 = sizeof(CT) == 4 && m.P % 4 == 0 && reinterpret_cast<uintptr_t>(J) % 16 == 0;
     auto by_tw = [&](auto nvc) {
         constexpr int NV = decltype(nvc)::value;
-        if constexpr (sizeof(CT) == 4 && NV <= 6) {  // 4 (NV - 1) TA registers: spills past NV = 6
-            if (v4) {
-                go(k_jac_stiff<NV, CT, 4>);
+        if constexpr (sizeof(CT) == 4 && NV <= 4) {
+            if (S.node_build) {
+                if (v4) go(k_jac_stiff<NV, CT, 4, true>);
+                else if (v2) go(k_jac_stiff<NV, CT, 2, true>);
+                else go(k_jac_stiff<NV, CT, 1, true>);
                 return;
             }
         }
-        if (v2) go(k_jac_stiff<NV, CT, 2>);
-        else go(k_jac_stiff<NV, CT, 1>);
+        if constexpr (sizeof(CT) == 4 && NV <= 6) {  // 4 (NV - 1) TA registers: spills past NV = 6
+            if (v4) {
+                go(k_jac_stiff<NV, CT, 4, false>);
+                return;
+            }
+        }
+        if (v2) go(k_jac_stiff<NV, CT, 2, false>);
+        else go(k_jac_stiff<NV, CT, 1, false>);
     };
     switch (m.nv) {
         case 3: by_tw(std::integral_constant<int, 3>()); break;
@@ -717,7 +805,9 @@ static void build_stiff_plan(Context &c, int dt) {
         tnodes.insert(tnodes.end(), v.begin(), v.end());
         nptr.push_back((int32_t)tnodes.size());
     }
-    const size_t stage = (size_t)nl_tile * row_bytes;
+    // node-wise table build (kNS nodes per electrode) or the general one (a row per node)
+    S.node_build = dt == 1 && NV <= 4 && nl_tile <= 32;
+    const size_t stage = S.node_build ? ((size_t)(c.nE + 1) * kNS * 8 + 15) / 16 * 16 : (size_t)nl_tile * row_bytes;
     if (kStiffSmem < fixed + stage + 2 * per_dip) return;
     const size_t tab_cap = (kStiffSmem - fixed - stage) / 16 * 16;
     const std::vector<int32_t> &ab = c.abmn_h;
