@@ -199,6 +199,16 @@ struct JacStiff {
     DBuf<uint8_t> d_lidx;
 };
 
+// Plan of the wavenumber-outermost Jacobian kernel (TW = 0: none): tile width,
+// data chunks with their local dipoles (electrode nE: at infinity) and every
+// datum's dipole pair (ia | im << 16).
+struct JacWave {
+    int TW = 0, KB = 1, nchunks = 0;  // KB: wavenumbers at a time
+    size_t smem = 0;
+    DBuf<int32_t> d_chunks, d_dipa, d_dipm;
+    DBuf<uint32_t> d_pairs;
+};
+
 // Learned preconditioner (learned.cu): graph of the system matrix, network
 // weights, activations of every layer and the training buffers.  bf16
 // tensors are stored as uint16_t.
@@ -301,6 +311,7 @@ struct Context {
     DBuf<int32_t> d_dip_a, d_dip_m, d_data_dip;  // nA x 2, nM x 2, D x 2 (ia, im)
     JacTiles jtiles[2];                          // FP64 and FP32 tables
     JacStiff jstiff[2];                          // stiffness-only plans (FP64, FP32 J)
+    JacWave jwave[2];                            // wavenumber-outermost plans (FP64, FP32 J)
     DBuf<float2> d_xhl;                          // FP32 J: potentials split into (hi, lo)
     bool jac_ready = false;
     DBuf<char> d_jscale;                         // per-datum / per-parameter scales

@@ -191,6 +191,142 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
+// asynchronous 8-byte global -> shared copy (both addresses 8-byte aligned)
+__device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s), "l"(gmem) : "memory");
+}
+
+// The same sums with the wavenumbers outermost, for parameters of at most
+// kWCells cells: a block takes TW consecutive parameters and one chunk of data
+// and keeps the sums of its (datum, parameter) pairs in registers, kWOut per
+// thread.  For each cell of the parameters and each batch of KB wavenumbers it
+// holds U and V = w_k (K + k^2 M) U of every electrode, forms the two dipole
+// tables of these wavenumbers alone, and adds nv-term products per pair; the
+// next batch's potentials arrive by cp.async in a second buffer meanwhile.
+// k_jacobian holds the tables of all wavenumbers at once: on a 72-electrode line
+// (18 wavenumbers, 1330 distinct dipoles) one cell per block and five chunks
+// were left, bound by shared-memory conflicts and rebuilt tables.  Bound here:
+// the FP64 pipe, nv operations per distinct dipole and per pair for each
+// wavenumber and cell.  FP64 J: that line 44 -> 21.8 ms, 41
+// electrodes (488 data, 76 dipoles) 0.74 -> 0.54; four cells per parameter (H2
+// forward mesh) 5.4 -> 2.0 ms, eight (3-D, 5336 data) 97 -> 20 ms.
+constexpr int kWT = 512;     // threads
+template <typename CT> constexpr int kWOut = sizeof(CT) == 4 ? 32 : 16;  // pairs per thread (32 registers)
+constexpr int kWCells = 8;   // cells per parameter, at most (the children of an H2 refinement)
+
+// data chunk: data [d0, d1), local dipoles and their offsets
+struct WaveChunk {
+    int32_t d0, d1, nA, nM, off_a, off_m, pad[2];
+};
+
+template <int NV, typename CT, int TW>
+__global__ void __launch_bounds__(kWT, 2)
+    k_jac_wave(const WaveChunk *__restrict__ chunks, const int32_t *__restrict__ dipa, const int32_t *__restrict__ dipm,
+               const uint32_t *__restrict__ pairs, const int32_t *__restrict__ pcell_ptr,
+               const int32_t *__restrict__ pcell, const int32_t *__restrict__ cells, const double *__restrict__ K,
+               const double *__restrict__ M, const double *__restrict__ kv, const double *__restrict__ w, int nK, int KB,
+               int nE, int64_t Rpad, const double *__restrict__ pot, const CT *__restrict__ scale_d,
+               const CT *__restrict__ scale_p, int64_t P, CT *__restrict__ J) {
+    extern __shared__ __align__(16) unsigned char wave_smem[];
+    const WaveChunk ch = chunks[blockIdx.y];
+    const int E1 = nE + 1;  // electrode nE: at infinity, zero potential
+    const int uk = NV * E1 * TW, sk = NV * NV * TW, tk = (ch.nA + ch.nM) * NV * TW;  // one wavenumber's entries
+    double *U = reinterpret_cast<double *>(wave_smem), *V = U + (size_t)2 * KB * uk, *S = V + (size_t)KB * uk;
+    CT *T = reinterpret_cast<CT *>(S + (size_t)KB * sk);  // per wavenumber TA, then TM
+    const int64_t p0 = (int64_t)blockIdx.x * TW;
+    const int c = threadIdx.x % TW, g = threadIdx.x / TW;  // this thread's parameter and first datum
+    constexpr int G = kWT / TW;
+    const int nd = ch.d1 - ch.d0;
+    constexpr int NO = kWOut<CT>;
+    CT acc[NO];
+#pragma unroll
+    for (int t = 0; t < NO; t++) acc[t] = 0;
+    int most = 0;  // cells of the tile's longest parameter
+    for (int64_t p = p0; p < P && p < p0 + TW; p++) most = max(most, pcell_ptr[p + 1] - pcell_ptr[p]);
+    const int nb = (nK + KB - 1) / KB, steps = most * nb;
+    auto cell_of = [&](int q, int cc) -> int64_t {
+        const int64_t p = p0 + cc;
+        if (p >= P) return -1;
+        const int32_t o = pcell_ptr[p] + q;
+        return o < pcell_ptr[p + 1] ? pcell[o] : -1;
+    };
+    // potentials of step (cell q, batch b) into its buffer; the column of the
+    // electrode at infinity and absent cells are zero
+    auto stage = [&](int step) {
+        const int q = step / nb, k0 = (step - q * nb) * KB, kn = min(KB, nK - k0);
+        double *dst = U + (size_t)(step & 1) * KB * uk;
+        for (int t = threadIdx.x; t < kn * NV * TW * E1; t += kWT) {
+            const int e = t % E1, r = t / E1, kk = r % kn, ic = r / kn, i = ic % NV, cc = ic / NV;
+            const int64_t cl = cell_of(q, cc);
+            double *o = dst + (size_t)kk * uk + (i * E1 + e) * TW + cc;
+            if (cl >= 0 && e < nE) cp_async8(o, pot + (int64_t)cells[cl * NV + i] * Rpad + (int64_t)(k0 + kk) * nE + e);
+            else *o = 0.0;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (steps) stage(0);
+    for (int step = 0; step < steps; step++) {
+        const int q = step / nb, k0 = (step - q * nb) * KB, kn = min(KB, nK - k0);
+        const double *Ub = U + (size_t)(step & 1) * KB * uk;
+        for (int t = threadIdx.x; t < kn * sk; t += kWT) {
+            const int cc = t % TW, r = t / TW, ij = r % (NV * NV), kk = r / (NV * NV);
+            const int64_t cl = cell_of(q, cc);
+            const double k = kv[k0 + kk];
+            S[t] = cl >= 0 ? w[k0 + kk] * fma(M[cl * NV * NV + ij], k * k, K[cl * NV * NV + ij]) : 0.0;
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // U and S of this step; the other U buffer was last read before the previous pair phase
+        if (step + 1 < steps) stage(step + 1);
+        for (int t = threadIdx.x; t < kn * uk; t += kWT) {
+            const int cc = t % TW, r = t / TW, kk = r / (NV * E1), ie = r - kk * NV * E1, i = ie / E1, e = ie - i * E1;
+            const double *Uk = Ub + (size_t)kk * uk, *Sk = S + (size_t)kk * sk;
+            double v = 0.0;
+#pragma unroll
+            for (int j = 0; j < NV; j++) v = fma(Sk[(i * NV + j) * TW + cc], Uk[(j * E1 + e) * TW + cc], v);
+            V[t] = v;
+        }
+        __syncthreads();
+        for (int t = threadIdx.x; t < kn * (ch.nA + ch.nM) * TW; t += kWT) {
+            const int cc = t % TW, r = t / TW, kk = r / (ch.nA + ch.nM), dp = r - kk * (ch.nA + ch.nM);
+            const bool isA = dp < ch.nA;
+            const int32_t *dd = isA ? dipa + 2 * (ch.off_a + dp) : dipm + 2 * (ch.off_m + dp - ch.nA);
+            const int a = dd[0], b = dd[1];
+            const double *src = (isA ? V : Ub) + (size_t)kk * uk;
+            CT *dst = T + (size_t)kk * tk + (size_t)dp * NV * TW + cc;
+#pragma unroll
+            for (int i = 0; i < NV; i++) dst[i * TW] = (CT)(src[(i * E1 + a) * TW + cc] - src[(i * E1 + b) * TW + cc]);
+        }
+        __syncthreads();
+        const CT *TA = T + c, *TM = T + (size_t)ch.nA * NV * TW + c;
+#pragma unroll
+        for (int t = 0; t < NO; t++) {
+            const int d = g + t * G;
+            if (d < nd) {
+                const uint32_t pr = pairs[ch.d0 + d];
+                const CT *ta = TA + (size_t)(pr & 0xffffu) * NV * TW, *tm = TM + (size_t)(pr >> 16) * NV * TW;
+                CT v = acc[t];
+                for (int kk = 0; kk < kn; kk++, ta += tk, tm += tk)
+#pragma unroll
+                    for (int i = 0; i < NV; i++) v = fma(ta[i * TW], tm[i * TW], v);
+                acc[t] = v;
+            }
+        }
+    }
+    const int64_t p = p0 + c;
+    if (p >= P) return;
+    const CT sp = scale_p ? scale_p[p] : (CT)1;
+#pragma unroll
+    for (int t = 0; t < NO; t++) {
+        const int d = g + t * G;
+        if (d < nd) {
+            CT v = acc[t];
+            if (scale_p) v = (v * scale_d[ch.d0 + d]) * sp;
+            J[(int64_t)(ch.d0 + d) * P + p] = v;
+        }
+    }
+}
+
 // scale_d[d] = kfac[d], scale_p[p] = 1 / model[p]^2 in the compute type
 template <typename CT>
 __global__ void k_jac_scales(int64_t D, int64_t P, const double *__restrict__ kfac,
@@ -285,11 +421,6 @@ template <> __device__ __forceinline__ double record_scale<double>(int4 m) {
     return __hiloint2double(m.w, m.z);
 }
 
-// asynchronous 8-byte global -> shared copy (both addresses 8-byte aligned)
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s), "l"(gmem) : "memory");
-}
 // asynchronous 16-byte global -> shared copy (both addresses 16-byte aligned)
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -658,11 +789,38 @@ void launch_stiff(Context &c, bool scaled, const CT *sp, CT *J, int dtype, cudaS
 }
 
 template <typename CT>
+void launch_wave(Context &c, const CT *sd, const CT *sp, CT *J, int dtype, cudaStream_t s) {
+    MeshData &m = c.mesh;
+    JacWave &W = c.jwave[dtype];
+    auto go = [&](auto kern, int TW) {
+        // always the same limit: contexts may launch from several host threads
+        ERTGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudgetLarge));
+        kern<<<dim3((unsigned)ceil_div(m.P, TW), (unsigned)W.nchunks), kWT, W.smem, s>>>(
+            reinterpret_cast<const WaveChunk *>(W.d_chunks.p), W.d_dipa.p, W.d_dipm.p, W.d_pairs.p, m.d_pcell_ptr.p,
+            m.d_pcell.p, m.d_cells.p, m.d_K.p, m.d_M.p, c.d_k.p, c.d_w.p, c.nK, W.KB, c.nE, c.Rpad, c.d_x.p, sd, sp, m.P,
+            J);
+        ERTGB_CUDA(cudaGetLastError());
+    };
+    auto by_tw = [&](auto nvc) {
+        constexpr int NV = decltype(nvc)::value;
+        if (W.TW == 8) go(k_jac_wave<NV, CT, 8>, 8);
+        else if (W.TW == 4) go(k_jac_wave<NV, CT, 4>, 4);
+        else go(k_jac_wave<NV, CT, 2>, 2);
+    };
+    switch (m.nv) {
+        case 3: by_tw(std::integral_constant<int, 3>()); break;
+        case 4: by_tw(std::integral_constant<int, 4>()); break;
+        case 6: by_tw(std::integral_constant<int, 6>()); break;
+        default: by_tw(std::integral_constant<int, 10>()); break;
+    }
+}
+
+template <typename CT>
 void launch(Context &c, const double *model, CT *J, int dtype, cudaStream_t s) {
     MeshData &m = c.mesh;
     JacTiles &T = c.jtiles[dtype];
     const int ntiles = (int)T.tile_p.size() - 1;
-    if (ntiles <= 0) return;
+    if (ntiles <= 0 && !c.jwave[dtype].TW) return;
     if (c.nK > 64) throw Error(ERTGB_BAD_INPUT, "Jacobian supports at most 64 wavenumbers");
     const int TW = T.max_cells, G = T.stage_cells;
     const size_t uv = (size_t)c.nK * m.nv * (c.nE + 1);
@@ -679,6 +837,10 @@ void launch(Context &c, const double *model, CT *J, int dtype, cudaStream_t s) {
     }
     if (c.jstiff[dtype].ok) {
         launch_stiff<CT>(c, sd != nullptr, sp, J, dtype, s);
+        return;
+    }
+    if (c.jwave[dtype].TW) {
+        launch_wave<CT>(c, sd, sp, J, dtype, s);
         return;
     }
     auto go = [&](auto kern) {
@@ -889,6 +1051,81 @@ static void build_stiff_plan(Context &c, int dt) {
     S.ok = true;
 }
 
+// Plan of the wavenumber-outermost kernel: tile width and data chunks of at most
+// its pairs in registers and its dipoles in the shared memory that leaves two
+// blocks per SM, then as many wavenumbers at a time as still fit.  A wider tile
+// restages the electrodes more often (fewer dipoles per chunk), a narrower one
+// stores J in shorter runs: 8, 4, then 2 parameters (32 bytes of FP64 J from 4
+// on) as long as a chunk holds a quarter of the scheme's dipoles or 256 of them
+// and the tiles fill the chip twice.
+static void build_wave_plan(Context &c, int dt) {
+    JacWave &W = c.jwave[dt];
+    W.TW = 0;
+    MeshData &m = c.mesh;
+    if (c.D == 0 || m.P == 0 || (m.nv != 3 && m.nv != 4 && m.nv != 6 && m.nv != 10)) return;
+    for (int64_t p = 0; p < m.P; p++)
+        if (m.pcell_ptr[p + 1] - m.pcell_ptr[p] > kWCells) return;
+    const size_t sz = dt == 0 ? 8 : 4;
+    // shared memory of one wavenumber: two buffers of U, V and S; a dipole's table row
+    auto fixed = [&](int tw) { return sizeof(double) * (size_t)tw * m.nv * (3 * (c.nE + 1) + m.nv); };
+    auto row = [&](int tw) { return (size_t)tw * m.nv * sz; };
+    int cap = 0;
+    for (int tw : {8, 4, 2}) {
+        if (fixed(tw) >= kSmemBudget) continue;
+        const int fit = (int)std::min<size_t>(65535, (kSmemBudget - fixed(tw)) / row(tw));
+        if (fit < 2) continue;
+        W.TW = tw;
+        cap = fit;
+        if (fit >= std::min((c.nA + c.nM + 3) / 4, 256) && ceil_div(m.P, tw) >= 304) break;
+    }
+    if (!W.TW) return;
+    const std::vector<int32_t> &ab = c.abmn_h;
+    auto col = [&](int32_t e) { return e < 0 ? c.nE : e; };
+    std::vector<WaveChunk> chunks;
+    std::vector<int32_t> dipa, dipm;
+    std::vector<uint32_t> pairs;
+    const int64_t most = (int64_t)kWT / W.TW * (dt == 0 ? kWOut<double> : kWOut<float>);
+    size_t dips = 0;
+    for (int64_t d = 0; d < c.D;) {
+        std::map<std::pair<int32_t, int32_t>, int32_t> amap, mmap;
+        WaveChunk ch{};
+        ch.d0 = (int32_t)d;
+        ch.off_a = (int32_t)(dipa.size() / 2);
+        ch.off_m = (int32_t)(dipm.size() / 2);
+        for (; d < c.D && d - ch.d0 < most; d++) {
+            const int32_t *q = &ab[4 * d];
+            const int add = (amap.count({q[0], q[1]}) ? 0 : 1) + (mmap.count({q[2], q[3]}) ? 0 : 1);
+            if ((int)(amap.size() + mmap.size()) + add > cap) break;
+            const auto ia = amap.emplace(std::make_pair(q[0], q[1]), (int32_t)amap.size());
+            if (ia.second) dipa.insert(dipa.end(), {col(q[0]), col(q[1])});
+            const auto im = mmap.emplace(std::make_pair(q[2], q[3]), (int32_t)mmap.size());
+            if (im.second) dipm.insert(dipm.end(), {col(q[2]), col(q[3])});
+            pairs.push_back((uint32_t)ia.first->second | ((uint32_t)im.first->second << 16));
+        }
+        ch.d1 = (int32_t)d;
+        ch.nA = (int32_t)amap.size();
+        ch.nM = (int32_t)mmap.size();
+        dips = std::max(dips, amap.size() + mmap.size());
+        chunks.push_back(ch);
+    }
+    if (chunks.size() > 65535) {
+        W.TW = 0;
+        return;
+    }
+    W.nchunks = (int)chunks.size();
+    const size_t one = fixed(W.TW) + dips * row(W.TW);
+    W.KB = (int)std::min<size_t>((size_t)c.nK, std::max<size_t>(1, kSmemBudget / one));
+    W.KB = (int)ceil_div(c.nK, ceil_div(c.nK, W.KB));  // even batches
+    W.smem = one * W.KB;
+    std::vector<int32_t> cw(chunks.size() * sizeof(WaveChunk) / sizeof(int32_t));
+    std::memcpy(cw.data(), chunks.data(), cw.size() * sizeof(int32_t));
+    W.d_chunks.upload(cw, c.stream);
+    W.d_dipa.upload(dipa, c.stream);
+    W.d_dipm.upload(dipm, c.stream);
+    W.d_pairs.upload(pairs, c.stream);
+    ERTGB_CUDA(cudaStreamSynchronize(c.stream));  // host lists are freed on return
+}
+
 // Parameter -> cells and the Jacobian tiles of both table precisions
 // (consecutive parameters with at most TW cells per tile).
 void build_jacobian_tiles(Context &c) {
@@ -942,11 +1179,15 @@ void build_jacobian_tiles(Context &c) {
         }
         T.d_tile_p.upload(T.tile_p, c.stream);
     }
-    for (int dt = 0; dt < 2; dt++) build_stiff_plan(c, dt);
+    for (int dt = 0; dt < 2; dt++) {
+        c.jwave[dt].TW = 0;
+        build_stiff_plan(c, dt);
+        if (!c.jstiff[dt].ok) build_wave_plan(c, dt);
+    }
 }
 
 void jacobian(Context &c, const double *model, int n_model, void *J, int dtype, cudaStream_t s) {
-    if (c.jtiles[dtype].max_cells == 0 && !c.jstiff[dtype].ok)
+    if (c.jtiles[dtype].max_cells == 0 && !c.jstiff[dtype].ok && !c.jwave[dtype].TW)
         throw Error(ERTGB_BAD_INPUT, "Jacobian tables of one cell exceed shared memory "
                                      "(too many wavenumbers x distinct dipoles)");
     const double *mdl = (n_model == c.mesh.P) ? model : nullptr;
@@ -956,7 +1197,7 @@ void jacobian(Context &c, const double *model, int n_model, void *J, int dtype, 
 
 void profile_jacobian(Context &c, int reps, void *J, int dtype, double *ms, double *bytes, double *flops) {
     if (!c.have_pot) throw Error(ERTGB_STATE, "profile needs a completed response");
-    if (c.jtiles[dtype].max_cells == 0 && !c.jstiff[dtype].ok)
+    if (c.jtiles[dtype].max_cells == 0 && !c.jstiff[dtype].ok && !c.jwave[dtype].TW)
         throw Error(ERTGB_BAD_INPUT, "no Jacobian plan for this scheme");
     MeshData &m = c.mesh;
     cudaStream_t s = c.stream;
