@@ -377,14 +377,12 @@ __global__ void k_jac_scales(int64_t D, int64_t P, const double *__restrict__ kf
 //
 // FP32 J of P1 cells with at most 32 distinct nodes per tile (FB): the potential
 // rows are staged electrode by electrode (kNS nodes each), and a warp builds a
-// table row with its lanes first as nodes, then as slots: the dipole's
-// difference u_a - u_b at every node as an error-free FP32 pair (Knuth's
-// two-sum on the hi parts, its error added to the lo difference), handed to the
-// slots by shuffles, and K_c from registers.  The general build reads every
-// node of every slot for both electrodes, 8 strided 8-byte loads and 9 of K_c
-// against 2 contiguous ones and 8 shuffles; with 2940 distinct dipoles
-// (box_3d_large, ten chunks per tile) it was five sixths of the kernel: 21.3 ->
-// 14.8 ms, box_3d (1200 dipoles) 3.30 -> 2.97 ms, 23k nodes 1.16 -> 0.92 ms.
+// table row with its lanes first as nodes, loading u_a and u_b of the dipole
+// contiguously, then as slots, fetching their nodes' pairs by shuffles, with
+// K_c in registers.  The general build reads every node of every slot for both
+// electrodes, 8 strided 8-byte loads and 9 of K_c; with 2940 distinct dipoles
+// (box_3d_large, ten chunks per tile) it was five sixths of the kernel.  Same
+// operations in the same order, so the two builds give the same J bit for bit.
 // ---------------------------------------------------------------------------
 
 constexpr int kSJT = 1024;  // threads of the stiffness kernel (one block per SM)
@@ -532,7 +530,8 @@ __global__ void __launch_bounds__(kSJT, 1)
                 const bool full = ln[0] != 0xff;
                 OT Kr[NM1 * NM1];
 #pragma unroll
-                for (int i = 0; i < NM1 * NM1; i++) Kr[i] = Ks[lane * NM1 * NM1 + i] * sps[lane];
+                for (int i = 0; i < NM1 * NM1; i++) Kr[i] = Ks[lane * NM1 * NM1 + i];
+                const OT fs = sps[lane];
                 const int ndip = cd.nA + cd.nM;
                 for (int first = warp; first < ndip; first += 32 * NW) {
                     // lane k holds the electrodes of the warp's k-th dipole
@@ -552,15 +551,15 @@ __global__ void __launch_bounds__(kSJT, 1)
                             ua = Us[a * kNS + lane];
                             ub = Us[b * kNS + lane];
                         }
-                        const float dh = ua.x - ub.x, t = dh - ua.x;
-                        const float dl = ((ua.x - (dh - t)) + (-ub.x - t)) + (ua.y - ub.y);
-                        const float h0 = __shfl_sync(0xffffffffu, dh, ln[0]), l0 = __shfl_sync(0xffffffffu, dl, ln[0]);
+                        auto at = [&](float2 u, int l) {
+                            return make_float2(__shfl_sync(0xffffffffu, u.x, l), __shfl_sync(0xffffffffu, u.y, l));
+                        };
+                        const float2 a0 = at(ua, ln[0]), b0 = at(ub, ln[0]);
                         OT gv[NM1];
 #pragma unroll
                         for (int j = 0; j < NM1; j++) {
-                            const float h = __shfl_sync(0xffffffffu, dh, ln[j + 1]);
-                            const float l = __shfl_sync(0xffffffffu, dl, ln[j + 1]);
-                            gv[j] = full ? (h - h0) + (l - l0) : (OT)0;
+                            const float g = dipole_shift(at(ua, ln[j + 1]), a0, at(ub, ln[j + 1]), b0);
+                            gv[j] = full ? g : (OT)0;
                         }
                         OT *dst = tabs + (size_t)dp * NM1 * TW + lane;
                         if (dp < cd.nA) {
@@ -569,7 +568,7 @@ __global__ void __launch_bounds__(kSJT, 1)
                                 OT sacc = 0;
 #pragma unroll
                                 for (int j = 0; j < NM1; j++) sacc = fma(Kr[i * NM1 + j], gv[j], sacc);
-                                dst[i * TW] = sacc;
+                                dst[i * TW] = sacc * fs;
                             }
                         } else {
 #pragma unroll
