@@ -14,8 +14,9 @@
 // The constraint matrix C (and its transpose) is CSR FP64.  Vectors and
 // scalars are FP64; the dot products are deterministic two-stage reductions
 // whose results the host reads every iteration (two syncs per iteration,
-// small against the two passes over J).  With an FP32 Jacobian the products
-// run in FP32 (per-thread partial sums) and are summed in FP64.
+// small against the two passes over J).  With an FP32 Jacobian whose rows start
+// 16-byte aligned (P a multiple of 4) the products run in FP32 (per-thread partial
+// sums) and are summed in FP64; with other P they run in FP64.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -29,29 +30,72 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kRowSeg = 16;  // row segments of the J^T products
 
+// J's element as FP64.  An FP32 value widens exactly without the FP64 pipe: its
+// bits shifted into place and the exponent rebased by 1023 - 127; subnormals are
+// first scaled to normal FP32 by 2^64.  Branch-free, so that no conversion
+// instruction is issued speculatively.
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ double widen(float v) {
+    const unsigned e = __float_as_uint(v) & 0x7f800000u;
+    const unsigned b = __float_as_uint(e == 0u ? v * 0x1p64f : v);
+    // exponent 0: zero stays zero; 255 (infinity, NaN): to 2047
+    unsigned bias = 0x38000000u;
+    bias = e == 0u ? ((b << 1) != 0u ? 0x34000000u : 0u) : bias;
+    bias = e == 0x7f800000u ? 0x70000000u : bias;
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + bias)), (int)(b << 29));
+}
+
+// FP64 arithmetic on J of either type.  The FP64 pipe bounds an FP32 J here (0.6e12
+// multiply-adds/s: 1.10 ms for 5336 x 124098 values against 0.39 ms of HBM), so
+// nothing but the multiply-adds may use it: with widen() in place of the
+// conversion instruction a pass takes 1.25 instead of 2.55 ms, bit for bit the
+// same.  kMulRows rows per block share the loads of x, whose L2 traffic is twice
+// that of an FP32 J with one row.
+constexpr int kMulRows = 2;
+
 template <typename T>
 __global__ void k_jmul(int64_t D, int64_t P, const T *__restrict__ J, const double *__restrict__ x,
                        const double *__restrict__ scale, double *__restrict__ y) {
     __shared__ double red[kThreads];
-    for (int64_t d = blockIdx.x; d < D; d += gridDim.x) {
-        const T *row = J + d * P;
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+    for (int64_t d = (int64_t)blockIdx.x * kMulRows; d < D; d += (int64_t)gridDim.x * kMulRows) {
+        const int nr = (int)min((int64_t)kMulRows, D - d);
+        const T *row[kMulRows];
+        double a[kMulRows][4];
+#pragma unroll
+        for (int r = 0; r < kMulRows; r++) {
+            row[r] = J + (d + min(r, nr - 1)) * P;  // past the end: the last row again, not stored
+#pragma unroll
+            for (int u = 0; u < 4; u++) a[r][u] = 0.0;
+        }
         int64_t p = threadIdx.x;
         for (; p + 3 * kThreads < P; p += 4 * kThreads) {
-            a0 = fma((double)row[p], x[p], a0);
-            a1 = fma((double)row[p + kThreads], x[p + kThreads], a1);
-            a2 = fma((double)row[p + 2 * kThreads], x[p + 2 * kThreads], a2);
-            a3 = fma((double)row[p + 3 * kThreads], x[p + 3 * kThreads], a3);
+            T v[kMulRows][4];
+            double xv[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                xv[u] = x[p + u * kThreads];
+#pragma unroll
+                for (int r = 0; r < kMulRows; r++) v[r][u] = row[r][p + u * kThreads];
+            }
+#pragma unroll
+            for (int r = 0; r < kMulRows; r++)
+#pragma unroll
+                for (int u = 0; u < 4; u++) a[r][u] = fma(widen(v[r][u]), xv[u], a[r][u]);
         }
-        for (; p < P; p += kThreads) a0 = fma((double)row[p], x[p], a0);
-        red[threadIdx.x] = (a0 + a1) + (a2 + a3);
-        __syncthreads();
-        for (int w = kThreads / 2; w > 0; w >>= 1) {
-            if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+        for (; p < P; p += kThreads)
+#pragma unroll
+            for (int r = 0; r < kMulRows; r++) a[r][0] = fma(widen(row[r][p]), x[p], a[r][0]);
+#pragma unroll
+        for (int r = 0; r < kMulRows; r++) {
+            red[threadIdx.x] = (a[r][0] + a[r][1]) + (a[r][2] + a[r][3]);
+            __syncthreads();
+            for (int w = kThreads / 2; w > 0; w >>= 1) {
+                if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+                __syncthreads();
+            }
+            if (threadIdx.x == 0 && r < nr) y[d + r] = scale ? red[0] * scale[d + r] : red[0];
             __syncthreads();
         }
-        if (threadIdx.x == 0) y[d] = scale ? red[0] * scale[d] : red[0];
-        __syncthreads();
     }
 }
 
@@ -65,11 +109,22 @@ __global__ void k_jtmul(int64_t D, int64_t P, const T *__restrict__ J, const dou
     if (p >= P) return;
     double a0 = 0.0, a1 = 0.0;
     int64_t d = d0;
-    for (; d + 1 < d1; d += 2) {
-        a0 = fma((double)J[d * P + p], y[d], a0);
-        a1 = fma((double)J[(d + 1) * P + p], y[d + 1], a1);
+    const T *col = J + p;
+    for (; d + 7 < d1; d += 8) {  // eight loads in flight
+        T v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = col[(d + u) * P];
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+            a0 = fma(widen(v[u]), y[d + u], a0);
+            a1 = fma(widen(v[u + 1]), y[d + u + 1], a1);
+        }
     }
-    if (d < d1) a0 = fma((double)J[d * P + p], y[d], a0);
+    for (; d + 1 < d1; d += 2) {
+        a0 = fma(widen(col[d * P]), y[d], a0);
+        a1 = fma(widen(col[(d + 1) * P]), y[d + 1], a1);
+    }
+    if (d < d1) a0 = fma(widen(col[d * P]), y[d], a0);
     part[(int64_t)blockIdx.y * P + p] = a0 + a1;
 }
 
@@ -283,6 +338,7 @@ int cgls_solve(const void *J, int dtype, int64_t D, int64_t P, int64_t NC, const
     const unsigned gP = cg.grid(P), gD = cg.grid(D), gC = cg.grid(std::max<int64_t>(NC, 1));
     const dim3 gT((unsigned)ceil_div(P, kThreads), kRowSeg);
     const unsigned gJ = (unsigned)std::min<int64_t>(D, 16 * cg.sms);
+    const unsigned gJ64 = (unsigned)ceil_div(D, kMulRows);  // hardware scheduling evens out the last wave
     DBuf<float> x32, y32;
     const bool fast32 = dtype == 1 && (P & 3) == 0;
     if (fast32) {
@@ -292,12 +348,12 @@ int cgls_solve(const void *J, int dtype, int64_t D, int64_t P, int64_t NC, const
     const dim3 gT4((unsigned)ceil_div(P / 4, kThreads), kRowSeg);
     auto Jx = [&](const double *xin, const double *scale, double *yout) {
         if (dtype == 0) {
-            k_jmul<double><<<gJ, kThreads, 0, s>>>(D, P, (const double *)J, xin, scale, yout);
+            k_jmul<double><<<gJ64, kThreads, 0, s>>>(D, P, (const double *)J, xin, scale, yout);
         } else if (fast32) {
             k_to32<<<gP, kThreads, 0, s>>>(P, xin, x32.p);
             k_jmul32<<<gJ, kThreads, 0, s>>>(D, P, (const float *)J, x32.p, scale, yout);
         } else {
-            k_jmul<float><<<gJ, kThreads, 0, s>>>(D, P, (const float *)J, xin, scale, yout);
+            k_jmul<float><<<gJ64, kThreads, 0, s>>>(D, P, (const float *)J, xin, scale, yout);
         }
     };
     auto JTy = [&](const double *yin, const double *div, double *out) {
