@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(kSJT, 1)
                                 OT sacc = 0;
 #pragma unroll
                                 for (int j = 0; j < NM1; j++) sacc = fma(Kr[i * NM1 + j], gv[j], sacc);
-                                dst[i * TW] = sacc * fs;
+                                dst[i * TW] = full ? sacc * fs : (OT)0;  // an empty slot's scale may not be finite
                             }
                         } else {
 #pragma unroll
