@@ -305,11 +305,15 @@ __global__ void __launch_bounds__(kWT, 2)
             if (d < nd) {
                 const uint32_t pr = pairs[ch.d0 + d];
                 const CT *ta = TA + (size_t)(pr & 0xffffu) * NV * TW, *tm = TM + (size_t)(pr >> 16) * NV * TW;
-                CT v = acc[t];
+                // FP32: the batch's products first, then one rounding into the sum.  With every
+                // product added to the running sum the error against the FP64 J was 1.08 (3-D,
+                // 2 to 8 cells per parameter) and 1.15 times (lines) that of k_jacobian; so it is
+                // 1.00 and 0.99 times
+                CT v = sizeof(CT) == 4 ? (CT)0 : acc[t];
                 for (int kk = 0; kk < kn; kk++, ta += tk, tm += tk)
 #pragma unroll
                     for (int i = 0; i < NV; i++) v = fma(ta[i * TW], tm[i * TW], v);
-                acc[t] = v;
+                acc[t] = sizeof(CT) == 4 ? acc[t] + v : v;
             }
         }
     }
@@ -1050,8 +1054,8 @@ static void build_stiff_plan(Context &c, int dt) {
     S.ok = true;
 }
 
-// Plan of the wavenumber-outermost kernel: tile width and data chunks of at most
-// its pairs in registers and its dipoles in the shared memory that leaves two
+// Plan of the wavenumber-outermost kernel (several wavenumbers; one where
+// tiles_faster says no): tile width and data chunks of at most its pairs in registers and its dipoles in the shared memory that leaves two
 // blocks per SM, then as many wavenumbers at a time as still fit.  A wider tile
 // restages the electrodes more often (fewer dipoles per chunk), a narrower one
 // stores J in shorter runs: 8, 4, then 2 parameters (32 bytes of FP64 J from 4
@@ -1125,6 +1129,21 @@ static void build_wave_plan(Context &c, int dt) {
     ERTGB_CUDA(cudaStreamSynchronize(c.stream));  // host lists are freed on return
 }
 
+// One wavenumber leaves the wave kernel no tables to save: where little work follows
+// a tile's staging, or FP32 arithmetic on few cells, k_jacobian's wider tiles win.
+// Wave against k_jacobian, 3-D P1, ms: FP64, two cells per parameter and 39 data
+// 0.86 : 0.72, three and 39 0.72 : 0.78; FP32, two cells 0.52 : 0.49 (86 data),
+// 0.69 : 0.63 (548), 2.61 : 2.08 (2353), three 0.68 : 0.60 (39), 2.55 : 2.48 (2353),
+// five 0.64 : 0.62 (39), six 0.63 : 0.64 (39), four 0.64 : 0.71 (548), 2.50 : 2.77 (2353).
+static bool tiles_faster(const Context &c, int dt) {
+    const JacTiles &T = c.jtiles[dt];
+    if (c.nK != 1 || T.max_cells == 0 || !T.chunks.empty()) return false;
+    int64_t most = 0;
+    for (int64_t p = 0; p < c.mesh.P; p++)
+        most = std::max<int64_t>(most, c.mesh.pcell_ptr[p + 1] - c.mesh.pcell_ptr[p]);
+    return c.D * most < (dt == 0 ? 100 : 200) || (dt == 1 && most <= 3);
+}
+
 // Parameter -> cells and the Jacobian tiles of both table precisions
 // (consecutive parameters with at most TW cells per tile).
 void build_jacobian_tiles(Context &c) {
@@ -1181,7 +1200,7 @@ void build_jacobian_tiles(Context &c) {
     for (int dt = 0; dt < 2; dt++) {
         c.jwave[dt].TW = 0;
         build_stiff_plan(c, dt);
-        if (!c.jstiff[dt].ok) build_wave_plan(c, dt);
+        if (!c.jstiff[dt].ok && !tiles_faster(c, dt)) build_wave_plan(c, dt);
     }
 }
 
