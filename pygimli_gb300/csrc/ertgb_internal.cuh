@@ -192,7 +192,7 @@ struct JacTiles {
 // ia | im << 16, geometric factor).
 struct JacStiff {
     bool ok = false, node_build = false;
-    int nchunks = 0, RS = 0;  // chunks, staged row length (columns)
+    int nchunks = 0, RS = 0;  // chunks, staged row length (columns; node-wise build: nodes)
     int64_t ntiles = 0;
     size_t tab_bytes = 0, stage_bytes = 0, smem = 0;
     DBuf<int32_t> d_pc, d_nptr, d_tnodes, d_dipa, d_dipm, d_chunks, d_meta;

@@ -380,7 +380,7 @@ __global__ void k_jac_scales(int64_t D, int64_t P, const double *__restrict__ kf
 // one 8-byte J store (two 4-byte stores when P is odd).
 //
 // FP32 J of P1 cells with at most 32 distinct nodes per tile (FB): the potential
-// rows are staged electrode by electrode (kNS nodes each), and a warp builds a
+// rows are staged electrode by electrode, and a warp builds a
 // table row with its lanes first as nodes, loading u_a and u_b of the dipole
 // contiguously, then as slots, fetching their nodes' pairs by shuffles, with
 // K_c in registers.  The general build reads every node of every slot for both
@@ -392,7 +392,6 @@ __global__ void k_jac_scales(int64_t D, int64_t P, const double *__restrict__ kf
 constexpr int kSJT = 1024;  // threads of the stiffness kernel (one block per SM)
 constexpr int kSTW = 32;    // parameters per tile
 constexpr int kNREC = 16;   // data records staged per warp batch
-constexpr int kNS = 33;     // FB: staged nodes per electrode (odd: rows of electrodes start 2 banks apart)
 
 // chunk descriptor: data range of the sorted records, dipoles and their offsets
 struct StiffChunk {
@@ -496,9 +495,9 @@ __global__ void __launch_bounds__(kSJT, 1)
         if constexpr (FB) {
             for (int q = threadIdx.x; q < nn * nE; q += kSJT) {
                 const int i = q / nE, e = q - i * nE;
-                cp_async8(Us + e * kNS + i, pot + (int64_t)tnodes[n0 + i] * Rpad + e);
+                cp_async8(Us + e * RS + i, pot + (int64_t)tnodes[n0 + i] * Rpad + e);
             }
-            for (int i = threadIdx.x; i < nn; i += kSJT) Us[nE * kNS + i] = ST{};
+            for (int i = threadIdx.x; i < nn; i += kSJT) Us[nE * RS + i] = ST{};
         } else {
             const int per = nE2 / 2;
             for (int q = threadIdx.x; q < nn * per; q += kSJT) {
@@ -552,8 +551,8 @@ __global__ void __launch_bounds__(kSJT, 1)
                         const int a = __shfl_sync(0xffffffffu, da, k), b = __shfl_sync(0xffffffffu, db, k);
                         float2 ua = make_float2(0.f, 0.f), ub = ua;
                         if (lane < nn) {
-                            ua = Us[a * kNS + lane];
-                            ub = Us[b * kNS + lane];
+                            ua = Us[a * RS + lane];
+                            ub = Us[b * RS + lane];
                         }
                         auto at = [&](float2 u, int l) {
                             return make_float2(__shfl_sync(0xffffffffu, u.x, l), __shfl_sync(0xffffffffu, u.y, l));
@@ -970,10 +969,15 @@ static void build_stiff_plan(Context &c, int dt) {
         tnodes.insert(tnodes.end(), v.begin(), v.end());
         nptr.push_back((int32_t)tnodes.size());
     }
-    // node-wise table build (kNS nodes per electrode) or the general one (a row per node)
-    S.node_build = dt == 1 && NV <= 4 && nl_tile <= 32;
-    const size_t stage = S.node_build ? ((size_t)(c.nE + 1) * kNS * 8 + 15) / 16 * 16 : (size_t)nl_tile * row_bytes;
-    if (kStiffSmem < fixed + stage + 2 * per_dip) return;
+    // Node-wise table build (NS nodes per electrode) or the general one (a row per
+    // node).  An odd NS spreads the staging's stores over the banks and may stage one
+    // node more than the tile has: with many electrodes that costs dipoles per chunk.
+    const int NS = nl_tile | 1;
+    const size_t rows = (size_t)nl_tile * row_bytes, nodes = ((size_t)(c.nE + 1) * NS * 8 + 15) / 16 * 16;
+    auto cap_of = [&](size_t st) { return kStiffSmem < fixed + st ? (size_t)0 : (kStiffSmem - fixed - st) / per_dip; };
+    S.node_build = dt == 1 && NV <= 4 && nl_tile <= 32 && cap_of(nodes) >= 2 && 4 * cap_of(nodes) >= 3 * cap_of(rows);
+    const size_t stage = S.node_build ? nodes : rows;
+    if (cap_of(stage) < 2) return;
     const size_t tab_cap = (kStiffSmem - fixed - stage) / 16 * 16;
     const std::vector<int32_t> &ab = c.abmn_h;
     auto col = [&](int32_t e) { return e < 0 ? c.nE : e; };
@@ -1033,7 +1037,7 @@ static void build_stiff_plan(Context &c, int dt) {
         }
         chunks.push_back(cd);
     }
-    S.RS = RS;
+    S.RS = S.node_build ? NS : RS;
     S.tab_bytes = (tab_max + 15) / 16 * 16;
     S.stage_bytes = stage;
     S.smem = S.tab_bytes + stage + fixed;

@@ -5,6 +5,8 @@ build, which runs on the same cells when their parameter numbers are scattered
 two builds do the same operations in the same order: equal to the last bit,
 also for parameters without a cell whose model value has no finite inverse
 square in FP32."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -12,6 +14,7 @@ from pygimli_gb300 import DataContainerERT, Mesh, create_box_mesh_3d
 from pygimli_gb300.data import geometricFactors, grid_line_scheme
 
 pytestmark = pytest.mark.gpu
+JACOBIAN32 = 4  # ERTGB_KERNEL_JACOBIAN32
 
 
 @pytest.fixture(scope="module")
@@ -75,3 +78,28 @@ def test_builds_agree(torch, empty, absent):
         assert int(without.sum()) == empty and bool((J[:, without] == 0).all())
         out.append(J[:, torch.from_numpy(mk).cuda()])
     assert bool(torch.isfinite(out[0]).all()) and torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("grid", [(20, 21), (29, 30), (30, 30)])
+def test_many_electrodes(torch, grid):
+    """The stiffness kernel's plan where the node-wise build leaves most of the
+    table space, about half of what the general one leaves (that one is taken)
+    and none.  The plan shows in the operation count of the kernel's profile."""
+    e = np.array([(x, y) for x in np.arange(grid[0]) * 4.0 for y in np.arange(grid[1]) * 4.0])
+    mesh = create_box_mesh_3d(e, h=4.0, para_depth=8.0, outer=120.0, growth=2.0)
+    nE, D, C = len(e), 300, mesh.cellCount()
+    assert most_nodes(mesh, np.arange(C)) <= 32
+    rng = np.random.default_rng(nE)
+    ab = np.array([rng.permutation(nE)[:4] for _ in range(D)], np.int32)
+    data = DataContainerERT(np.column_stack([e, np.zeros(nE)]), ab)
+    data.set("k", rng.uniform(1.0, 9.0, D))
+    f = operator(mesh, data, np.arange(C))
+    rho = np.exp(rng.normal(np.log(100.0), 0.5, C))
+    f.response(rho)
+    J, F = f.createJacobian(rho, dtype="float64"), f.createJacobian(rho, dtype="float32")
+    assert float(torch.linalg.vector_norm(F.double() - J) / torch.linalg.vector_norm(J)) <= 2e-6
+    ms, nbytes, flops = ctypes.c_double(), ctypes.c_double(), ctypes.c_double()
+    f._check(f._lib.ertgb_profile_kernel(f._ctx, JACOBIAN32, 1, ctypes.c_void_p(F.data_ptr()), ctypes.byref(ms),
+                                         ctypes.byref(nbytes), ctypes.byref(flops)))
+    nA, nM = len(np.unique(ab[:, :2], axis=0)), len(np.unique(ab[:, 2:], axis=0))
+    assert flops.value == C * ((nE + 1) * 3 + (nA + nM) * 9.0 + nA * 18.0) + D * C * 8.0
