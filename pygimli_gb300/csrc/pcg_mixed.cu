@@ -696,6 +696,8 @@ int pcg_solve_mixed(Context &c, cudaStream_t s) {
                     c.d_pnorm2.n >= (size_t)Rpad ? c.d_pnorm2.p : nullptr);
     ERTGB_CUDA(cudaGetLastError());
     c.stats.launches_response += 5;
+    // with coarse levels a stall belongs to its model: the next one starts in FP32 again
+    if (ml) c.fp64_k.clear();
     if ((int)c.fp64_k.size() == c.nK) {
         std::vector<int32_t> pre((size_t)Rpad, 0);
         int32_t n_pre = 0;
@@ -793,7 +795,7 @@ int pcg_solve_mixed(Context &c, cudaStream_t s) {
     ERTGB_CUDA(cudaMemcpyAsync(&h_stalled, cs.nstalled, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     ERTGB_CUDA(cudaStreamSynchronize(s));
     c.stats.stalled_columns = h_stalled;
-    if (status == ERTGB_OK) {  // wavenumbers with at least half of their columns stalled start in FP64 next time
+    if (status == ERTGB_OK && !ml) {  // wavenumbers with at least half of their columns stalled start in FP64 next time
         std::vector<int32_t> st((size_t)Rpad);
         ERTGB_CUDA(cudaMemcpyAsync(st.data(), cs.stalled, sizeof(int32_t) * Rpad, cudaMemcpyDeviceToHost, s));
         ERTGB_CUDA(cudaStreamSynchronize(s));

@@ -1,0 +1,60 @@
+"""A model whose columns stall in FP32 with coarse levels leaves no trace on the
+next one."""
+import numpy as np
+import pytest
+
+from pygimli_gb300 import DataContainerERT, create_box_mesh_3d
+from pygimli_gb300.data import geometricFactors, grid_line_scheme
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def torch():
+    t = pytest.importorskip("torch")
+    if not t.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from pygimli_gb300 import build
+    build.build()
+    return t
+
+
+@pytest.fixture(scope="module")
+def grid():
+    e = np.array([(x, y) for x in np.arange(12) * 4.0 for y in np.arange(8) * 4.0])
+    mesh = create_box_mesh_3d(e, h=4.0)
+    data = DataContainerERT(np.column_stack([e, np.zeros(len(e))]), grid_line_scheme((12, 8), "pd"))
+    data.set("k", geometricFactors(data, 3))
+    return mesh, data
+
+
+def operator(grid, **kw):
+    from pygimli_gb300 import ERTModelling
+    f = ERTModelling(maxIter=200000, precision="mixed", **kw)
+    f.setData(grid[1])
+    f.setMesh(grid[0], ignoreRegionManager=True)
+    return f
+
+
+def lognormal(mesh, sigma, seed):
+    return np.exp(np.random.default_rng(seed).normal(np.log(100.0), sigma, mesh.cellCount()))
+
+
+def bodies(mesh, factor):
+    c, rho = mesh.cellCenters(), lognormal(mesh, 1.0, 1)
+    rho[np.linalg.norm(c - [12.0, 8.0, -4.0], axis=1) < 4.0] = 100.0 / factor
+    rho[np.linalg.norm(c - [28.0, 16.0, -5.0], axis=1) < 4.0] = 100.0 * factor
+    return rho
+
+
+@pytest.mark.parametrize("precond", ["jacobi", "fsai"])
+def test_stall_is_not_carried_over(torch, grid, precond):
+    ordinary = lognormal(grid[0], 1.0, 9)
+    f = operator(grid, precond=precond)
+    first, its = f.response(ordinary), f.stats()["iterations"]
+    for _ in range(2):
+        f.response(bodies(grid[0], 1e9))
+        assert f.stats()["stalled_columns"] >= 48  # half of the sources and more
+        again, st = f.response(ordinary), f.stats()
+        assert st["stalled_columns"] == 0 and st["iterations"] == its
+        assert np.array_equal(first, again)
