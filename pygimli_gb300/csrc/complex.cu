@@ -841,7 +841,7 @@ __global__ void k_finish_ml_c(int64_t Rpad, int NB, double rtol2, const double *
         stalls += 1.0;
     }
     col[C_STALLS * Rpad + t] = stalls;
-    if (stalls >= 4.0) {
+    if (stalls >= kMlPatience) {
         active[t] = 0;
         stalled[t] = 1;
         atomicAdd(nstalled, 1);

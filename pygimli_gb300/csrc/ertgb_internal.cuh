@@ -471,6 +471,13 @@ void ml_cycle(Context &c, const MlBlock<float> &v, int NB, double *pz, cudaStrea
 bool ml_setup64(Context &c, const double *val, int64_t cols, cudaStream_t s);
 void ml_cycle64(Context &c, const MlBlock<double> &v, int NB, double *pz, cudaStream_t s);
 int ml_launches(const Context &c);
+// Intervals (of six iterations) without a tenth less residual before a column
+// counts as stalled with coarse levels; 4 x 64 iterations without.  On very rough
+// ground CG rests for a while: with 4 intervals half the columns of a log-normal
+// ground of sigma 5 went to the FP64 finish at 1e-6 (23k nodes, FSAI: 807 ms
+// against 58 so and 68 without coarse levels); waiting 64 costs where FP32 cannot
+// converge (bodies of 1e7 times either way: 243 ms, 153 so).
+constexpr double kMlPatience = 16.0;
 // band.cu: inverse of one SPD matrix of at most 112 rows, in place (one block)
 constexpr int kDenseMax = 112;
 void dense_inverse(double *A, int n, int32_t *bad, cudaStream_t s);

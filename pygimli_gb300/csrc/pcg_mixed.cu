@@ -559,7 +559,7 @@ __global__ void k_m_finish_ml(int64_t Rpad, int NB, double rtol2, const double *
         stalls += 1.0;
     }
     col[STALLS * Rpad + t] = stalls;
-    if (stalls >= 4.0) {
+    if (stalls >= kMlPatience) {
         cs.active[t] = 0;
         cs.stalled[t] = 1;
         atomicAdd(cs.nstalled, 1);

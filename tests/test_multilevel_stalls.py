@@ -1,5 +1,7 @@
-"""A model whose columns stall in FP32 with coarse levels leaves no trace on the
-next one."""
+"""Ground on which the FP32 phase of the mixed solver rests or stalls with
+coarse levels: a stalled model leaves no trace on the next one, and very rough
+ground converges in FP32 (384 to 1730 iterations with the single level, measured
+at 160 to 560 with coarse levels)."""
 import numpy as np
 import pytest
 
@@ -58,3 +60,11 @@ def test_stall_is_not_carried_over(torch, grid, precond):
         again, st = f.response(ordinary), f.stats()
         assert st["stalled_columns"] == 0 and st["iterations"] == its
         assert np.array_equal(first, again)
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+def test_rough_ground_converges_in_fp32(torch, grid, seed):
+    f = operator(grid, precond="fsai")
+    f.response(lognormal(grid[0], 5.0, seed))
+    st = f.stats()
+    assert st["stalled_columns"] == 0 and st["iterations"] <= 900 and st["max_rel_residual"] <= 1e-10, st
