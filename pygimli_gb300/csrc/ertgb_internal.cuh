@@ -403,7 +403,7 @@ void clean_fixed_rows(Context &c, double *vals, cudaStream_t s);
 void check_rho(Context &c, const double *rho_cell, cudaStream_t s);
 // pcg.cu
 // mask: warm start (x kept) on the columns with mask[t] != 0; nullptr = cold start, all columns
-int pcg_solve(Context &c, cudaStream_t s, const int32_t *mask = nullptr);
+int pcg_solve(Context &c, cudaStream_t s, const int32_t *mask = nullptr, bool coarse = false);
 // allocate pcg_solve's workspaces ahead (no allocation inside a later solve)
 void pcg_prepare(Context &c);
 void pcg_finish_init(dim3 g, dim3 b, cudaStream_t s, int64_t Rpad, int64_t R, int NB, const double *pa,

@@ -346,7 +346,7 @@ void pcg_prepare(Context &c) {
     c.d_part.alloc((size_t)NB * Rpad * 3);
 }
 
-int pcg_solve(Context &c, cudaStream_t s, const int32_t *mask) {
+int pcg_solve(Context &c, cudaStream_t s, const int32_t *mask, bool coarse) {
     if (c.precond == ERTGB_PRECOND_BAND && !mask) return band_solve(c, s);  // direct, no iterations
     MeshData &m = c.mesh;
     const int64_t n = m.n, Rpad = c.Rpad, R = c.R;
@@ -389,8 +389,8 @@ int pcg_solve(Context &c, cudaStream_t s, const int32_t *mask) {
     // IC(0) (plain FP64 solve only; the FP64 finish of the mixed solver keeps Jacobi)
     const bool ic0 = c.precond == ERTGB_PRECOND_IC0 && !mask;
     // coarse levels around Jacobi (3-D); the FP64 finish of the mixed solver's
-    // stalled columns keeps the single level
-    const bool ml = c.precond == ERTGB_PRECOND_JACOBI && c.precision == ERTGB_PRECISION_FP64 && !mask &&
+    // stalled columns has them where its FP32 phase had
+    const bool ml = (mask ? coarse : c.precond == ERTGB_PRECOND_JACOBI && c.precision == ERTGB_PRECISION_FP64) &&
                     ml_setup64(c, c.d_S.p, Rpad, s);
     const bool zform = ic0 || ml;  // z = M^-1 r is a product of its own
     const double *dv = zform ? nullptr : c.d_dinv.p;

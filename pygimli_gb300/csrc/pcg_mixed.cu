@@ -809,7 +809,7 @@ int pcg_solve_mixed(Context &c, cudaStream_t s) {
     if (status == ERTGB_OK && h_stalled > 0) {
         // FP64 PCG on the stalled columns, warm-started from their FP64 solution
         c.stats.iterations = 0;
-        return pcg_solve(c, s, cs.stalled);
+        return pcg_solve(c, s, cs.stalled, ml);
     }
     std::vector<int32_t> it_h(Rpad);
     std::vector<double> rn(Rpad), bn(Rpad);

@@ -1,7 +1,11 @@
 """Ground on which the FP32 phase of the mixed solver rests or stalls with
-coarse levels: a stalled model leaves no trace on the next one, and very rough
-ground converges in FP32 (384 to 1730 iterations with the single level, measured
-at 160 to 560 with coarse levels)."""
+coarse levels: a stalled model leaves no trace on the next one, very rough
+ground converges in FP32, and the FP64 finish of columns that FP32 cannot solve
+has the coarse levels too.
+
+Iteration bars: the single level needs 384 to 1730 FP32 iterations on the rough
+ground and 660 to 880 FP64 iterations in the finish; the coarse levels were
+measured at 160 to 560 and 50 to 150."""
 import numpy as np
 import pytest
 
@@ -68,3 +72,29 @@ def test_rough_ground_converges_in_fp32(torch, grid, seed):
     f.response(lognormal(grid[0], 5.0, seed))
     st = f.stats()
     assert st["stalled_columns"] == 0 and st["iterations"] <= 900 and st["max_rel_residual"] <= 1e-10, st
+
+
+@pytest.mark.parametrize("precond", ["jacobi", "fsai"])
+def test_finish_has_coarse_levels(torch, grid, precond):
+    f = operator(grid, precond=precond)
+    f.response(bodies(grid[0], 1e9))
+    st = f.stats()
+    assert st["stalled_columns"] >= 48 and st["iterations"] <= 400 and st["max_rel_residual"] <= 1e-10, st
+
+
+@pytest.mark.parametrize("ground", ["rough", "bodies"])
+def test_complex_finish_has_coarse_levels(torch, ground):
+    """Complex columns that stall in FP32; the single level needs 11000 and 950
+    iterations on these models."""
+    e = np.array([(x, y) for x in np.arange(9) * 4.0 for y in np.arange(7) * 4.0])
+    mesh = create_box_mesh_3d(e, h=4.0)
+    data = DataContainerERT(np.column_stack([e, np.zeros(len(e))]), grid_line_scheme((9, 7), "pd"))
+    data.set("k", geometricFactors(data, 3))
+    f = operator((mesh, data))
+    f.setComplex(True)
+    rho = lognormal(mesh, 5.0, 505) if ground == "rough" else bodies(mesh, 1e8)
+    ph = -0.03 * np.random.default_rng(1).uniform(0.2, 1.0, len(rho))
+    f.response(np.concatenate([rho * np.cos(ph), rho * np.sin(ph)]))
+    st = f.stats()
+    assert st["stalled_columns"] > 0 and st["max_rel_residual"] <= 1e-10
+    assert st["iterations"] <= (3000 if ground == "rough" else 500), st
