@@ -232,6 +232,18 @@ int ertgb_set_precision(ertgb_ctx *ctx, int precision);
  * leaves the preconditioner alone on the fine level, the plain PCG. */
 int ertgb_set_coarse_levels(ertgb_ctx *ctx, int on);
 
+/* Releases the device memory that a context keeps for speed only: the coarse
+ * levels and the blocks of the banded solve's cyclic reduction.  A response or
+ * Jacobian that runs out of memory does this by itself and goes on with the
+ * single-level solver or the serial band factor; a caller does it before an
+ * allocation of its own that does not fit.  The next response takes the memory
+ * again if it is free. */
+int ertgb_trim(ertgb_ctx *ctx);
+/* Limit, in bytes, on what the library buffers allocated by the calling thread
+ * may hold (below 0: none, the default); beyond it a call meets ERTGB_OOM as if
+ * the device were full.  used (may be null): what they hold now. */
+int ertgb_alloc_limit(int64_t bytes, int64_t *used);
+
 /* Forward response: DCMultiElectrodeModelling::response
  * (core/src/bert/dcfemmodelling.cpp:1085-1197) for a per-cell resistivity
  * (the result of mapERTModel, :1199-1218).  Writes n_data apparent

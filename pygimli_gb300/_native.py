@@ -60,6 +60,8 @@ SIGNATURES = {
     "ertgb_set_solver": (_ci, [_vp, _d, _ci, _ci]),
     "ertgb_set_precision": (_ci, [_vp, _ci]),
     "ertgb_set_coarse_levels": (_ci, [_vp, _ci]),
+    "ertgb_trim": (_ci, [_vp]),
+    "ertgb_alloc_limit": (_ci, [ctypes.c_int64, ctypes.POINTER(ctypes.c_int64)]),
     "ertgb_set_formulation": (_ci, [_vp, _ci]),
     "ertgb_set_extension": (_ci, [_vp, _ci, ctypes.c_int64, _vp, _vp, _vp, _vp, _vp, _ci]),
     "ertgb_response": (_ci, [_vp, _vp, _vp, _vp]),

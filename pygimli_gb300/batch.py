@@ -91,5 +91,14 @@ class BatchedERTModelling:
 
     def createJacobian(self, models, dtype="float64"):
         """Jacobians of every problem from the potentials of the last batched
-        response (list of device tensors)."""
-        return [f.createJacobian(m, dtype=dtype) for f, m in zip(self.fops, models)]
+        response (list of device tensors).  If one does not fit, the batch lets
+        go of what its operators keep for speed only."""
+        out = []
+        for f, m in zip(self.fops, models):
+            try:
+                out.append(f.createJacobian(m, dtype=dtype))
+            except _torch().cuda.OutOfMemoryError:
+                for g in self.fops:
+                    g.trim()
+                out.append(f.createJacobian(m, dtype=dtype))
+        return out

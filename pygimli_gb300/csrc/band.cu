@@ -599,17 +599,9 @@ int band_solve(Context &c, cudaStream_t s) {
     ERTGB_CUDA(cudaMemcpyAsync(c.d_x.p, c.d_r.p, sizeof(double) * n * c.Rpad, cudaMemcpyDeviceToDevice, s));
     const int B = (int)std::max<int64_t>(b, 8), N = (int)ceil_div(n, B);
     const size_t blk = (size_t)c.nK * N * B * B;
-    bool reduction = B <= kCrMax;
+    const bool reduction = B <= kCrMax && !c.lean;
     if (reduction) {
-        try {
-            c.d_band.alloc(4 * blk);
-        } catch (Error &e) {
-            if (e.code != ERTGB_OOM) throw;
-            cudaGetLastError();  // a failed allocation: the serial form needs a quarter of it
-            reduction = false;
-        }
-    }
-    if (reduction) {
+        c.d_band.alloc(4 * blk);
         const CrMat M{c.d_band.p, c.d_band.p + blk, c.d_band.p + 2 * blk, c.d_band.p + 3 * blk, N, B};
         ERTGB_CUDA(cudaMemsetAsync(M.D, 0, sizeof(double) * 2 * blk, s));
         k_cr_fill<<<(unsigned)std::min<int64_t>(ceil_div((int64_t)N * B * c.nK, kBandThreads), 4096), kBandThreads, 0,

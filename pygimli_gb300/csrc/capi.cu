@@ -48,6 +48,30 @@ template <class F> int guard(Context *c, F &&f) {
     }
 }
 
+// f, and once more without what only speed needs if it runs out of memory
+template <class F> void with_less(const std::vector<Context *> &cs, F &&f) {
+    try {
+        f();
+        return;
+    } catch (Error &e) {
+        if (e.code != ERTGB_OOM) throw;
+    }
+    cudaGetLastError();
+    struct Lean {
+        const std::vector<Context *> &cs;
+        explicit Lean(const std::vector<Context *> &v) : cs(v) {
+            for (Context *c : cs) {
+                trim(*c);
+                c->lean = true;
+            }
+        }
+        ~Lean() {
+            for (Context *c : cs) c->lean = false;
+        }
+    } lean(cs);
+    f();
+}
+
 void clear_reference(Context &c) {
     c.ref_elec = -1;
     c.ref_node = -1;
@@ -88,6 +112,20 @@ struct StreamJoin {
 };
 
 }  // namespace
+
+void ertgb::trim(Context &c) {
+    ERTGB_CUDA(cudaStreamSynchronize(c.stream));
+    Multilevel &M = c.mesh.ml;
+    M.levels.clear();
+    M.px.release();
+    M.pt.release();
+    M.pg.release();
+    M.tried = M.ok = false;
+    c.d_band.release();
+    c.d_z.release();
+    c.d_z32.release();
+    c.cx.Sre.release();
+}
 
 void ertgb::set_free_error(const std::string &msg) { g_free_error = msg; }
 
@@ -275,6 +313,59 @@ void do_jacobian(Context &c, const double *model, int n_model, void *J, int dtyp
     c.stats.ms_jacobian = elapsed(c, 4, 5);
     c.stats.launches_jacobian = 1;
     j.done();
+}
+
+int batch_response(std::vector<Context *> &cs, const double *const *rho, double *const *rhoa, ertgb_batch_info *info,
+                   void *stream) {
+    Context &c0 = *cs[0];
+    const int n = (int)cs.size();
+    for (Context *c : cs) {
+        if (c->rhs_align != 128) {
+            c->rhs_align = 128;
+            invalidate_derived(*c);
+        }
+        ensure_derived(*c);
+    }
+    // derived data (primary potentials, boundary terms, unit matrices) is
+    // built on each context's stream; the batch runs on the first one
+    for (Context *c : cs) ERTGB_CUDA(cudaStreamSynchronize(c->stream));
+    StreamJoin j(c0, stream);
+    cudaStream_t s = c0.stream;
+    ertgb_batch_info local{};
+    ertgb_batch_info *inf = info ? info : &local;
+    std::memset(inf, 0, sizeof(*inf));
+    ERTGB_CUDA(cudaEventRecord(c0.ev[0], s));
+    for (int i = 0; i < n; i++) {
+        Context &c = *cs[i];
+        c.have_pot = false;
+        c.stats = ertgb_stats{};
+        check_rho(c, rho[i], s);
+        c.d_rho_last = rho[i];
+        c.d_S.alloc((size_t)c.nK * c.mesh.nnz);
+        assemble_all(c, rho[i], c.d_S.p, s);
+        compute_source_rho(c, rho[i], s);
+        c.d_r.alloc((size_t)c.mesh.n * c.Rpad);
+        build_rhs(c, s);
+        compute_rhs_scale(c, s);
+        c.have_S = true;
+    }
+    ERTGB_CUDA(cudaEventRecord(c0.ev[1], s));
+    int stalled = 0;
+    const int status = batch_solve(cs, s, inf, &stalled);
+    inf->stalled_columns = stalled;
+    ERTGB_CUDA(cudaEventRecord(c0.ev[2], s));
+    for (int i = 0; i < n; i++) {
+        finish_potentials(*cs[i], s);
+        collect_response(*cs[i], rhoa[i], s);
+    }
+    ERTGB_CUDA(cudaEventRecord(c0.ev[3], s));
+    ERTGB_CUDA(cudaEventSynchronize(c0.ev[3]));
+    inf->ms_assemble = elapsed(c0, 0, 1);
+    inf->ms_solve = elapsed(c0, 1, 2);
+    inf->ms_collect = elapsed(c0, 2, 3);
+    for (Context *c : cs) c->have_pot = status == ERTGB_OK;
+    j.done();
+    return status;
 }
 
 }  // namespace
@@ -751,12 +842,26 @@ int ertgb_set_coarse_levels(ertgb_ctx *ctx, int on) {
     return guard(c, [&] { c->coarse_levels = on != 0; });
 }
 
+int ertgb_trim(ertgb_ctx *ctx) {
+    Context *c = reinterpret_cast<Context *>(ctx);
+    return guard(c, [&] {
+        ERTGB_CUDA(cudaSetDevice(c->device));
+        trim(*c);
+    });
+}
+
+int ertgb_alloc_limit(int64_t bytes, int64_t *used) {
+    g_alloc_limit = bytes;
+    if (used) *used = g_alloc_used;
+    return ERTGB_OK;
+}
+
 int ertgb_response(ertgb_ctx *ctx, const double *rho_cell_dev, double *rhoa_dev, void *stream) {
     Context *c = reinterpret_cast<Context *>(ctx);
     int status = ERTGB_OK;
     int rc = guard(c, [&] {
         ERTGB_REQUIRE(rho_cell_dev && rhoa_dev, "null buffer");
-        status = do_response(*c, rho_cell_dev, rhoa_dev, stream);
+        with_less({c}, [&] { status = do_response(*c, rho_cell_dev, rhoa_dev, stream); });
         if (status == ERTGB_NOT_CONVERGED) throw Error(ERTGB_NOT_CONVERGED, "PCG did not converge");
     });
     return rc;
@@ -768,9 +873,12 @@ int ertgb_response_host(ertgb_ctx *ctx, const double *rho_cell, double *rhoa) {
         ERTGB_REQUIRE(rho_cell && rhoa, "null buffer");
         if (!c->have_mesh || !c->have_scheme) throw Error(ERTGB_STATE, "mesh and scheme needed");
         ERTGB_CUDA(cudaSetDevice(c->device));
-        c->d_rho_tmp.upload(rho_cell, (size_t)c->mesh.C, c->stream);
-        c->d_rhoa.alloc((size_t)c->D);
-        int st = do_response(*c, c->d_rho_tmp.p, c->d_rhoa.p, nullptr);
+        int st = ERTGB_OK;
+        with_less({c}, [&] {
+            c->d_rho_tmp.upload(rho_cell, (size_t)c->mesh.C, c->stream);
+            c->d_rhoa.alloc((size_t)c->D);
+            st = do_response(*c, c->d_rho_tmp.p, c->d_rhoa.p, nullptr);
+        });
         ERTGB_CUDA(cudaMemcpyAsync(rhoa, c->d_rhoa.p, sizeof(double) * c->D, cudaMemcpyDeviceToHost, c->stream));
         ERTGB_CUDA(cudaStreamSynchronize(c->stream));
         if (st == ERTGB_NOT_CONVERGED) throw Error(ERTGB_NOT_CONVERGED, "PCG did not converge");
@@ -782,7 +890,7 @@ int ertgb_jacobian(ertgb_ctx *ctx, const double *model_dev, int n_model, void *J
     return guard(c, [&] {
         ERTGB_REQUIRE(J_dev, "null buffer");
         ERTGB_REQUIRE(n_model == 0 || model_dev, "null model");
-        do_jacobian(*c, model_dev, n_model, J_dev, dtype, stream);
+        with_less({c}, [&] { do_jacobian(*c, model_dev, n_model, J_dev, dtype, stream); });
     });
 }
 
@@ -798,8 +906,10 @@ int ertgb_jacobian_host(ertgb_ctx *ctx, const double *model, int n_model, void *
             md = c->d_model_tmp.p;
         }
         const size_t bytes = (size_t)c->D * c->mesh.P * (dtype == 0 ? 8 : 4);
-        c->d_J_tmp.alloc(bytes);
-        do_jacobian(*c, md, n_model, c->d_J_tmp.p, dtype, nullptr);
+        with_less({c}, [&] {
+            c->d_J_tmp.alloc(bytes);
+            do_jacobian(*c, md, n_model, c->d_J_tmp.p, dtype, nullptr);
+        });
         copy_to_host(*c, J, c->d_J_tmp.p, bytes);
         ERTGB_CUDA(cudaStreamSynchronize(c->stream));
     });
@@ -944,11 +1054,13 @@ int ertgb_assemble(ertgb_ctx *ctx, const double *rho, void *stream) {
     return guard(c, [&] {
         ERTGB_REQUIRE(rho, "null resistivity");
         StreamJoin j(*c, stream);
-        ensure_derived(*c);
-        c->have_pot = false;
-        check_rho(*c, rho, c->stream);
-        c->d_S.alloc((size_t)c->nK * c->mesh.nnz);
-        assemble_all(*c, rho, c->d_S.p, c->stream);
+        with_less({c}, [&] {
+            ensure_derived(*c);
+            c->have_pot = false;
+            check_rho(*c, rho, c->stream);
+            c->d_S.alloc((size_t)c->nK * c->mesh.nnz);
+            assemble_all(*c, rho, c->d_S.p, c->stream);
+        });
         c->have_S = true;
         j.done();
     });
@@ -960,7 +1072,7 @@ int ertgb_lp_forward(ertgb_ctx *ctx, const float *theta, float *G, void *stream)
         ERTGB_REQUIRE(theta, "null weights");
         if (!c->have_S) throw Error(ERTGB_STATE, "no assembled matrices (ertgb_assemble or a response first)");
         StreamJoin j(*c, stream);
-        lp_forward(*c, theta, c->stream);
+        with_less({c}, [&] { lp_forward(*c, theta, c->stream); });
         if (G)
             ERTGB_CUDA(cudaMemcpyAsync(G, c->d_G32.p, (size_t)c->lp.nL * c->nK * sizeof(float),
                                        cudaMemcpyDeviceToDevice, c->stream));
@@ -974,7 +1086,7 @@ int ertgb_lp_loss_grad(ertgb_ctx *ctx, const float *theta, float *grad, double *
         ERTGB_REQUIRE(theta && loss, "null weights or loss");
         if (!c->have_S) throw Error(ERTGB_STATE, "no assembled matrices (ertgb_assemble or a response first)");
         StreamJoin j(*c, stream);
-        *loss = lp_loss_grad(*c, theta, grad, c->stream);
+        with_less({c}, [&] { *loss = lp_loss_grad(*c, theta, grad, c->stream); });
         j.done();
     });
 }
@@ -1000,7 +1112,7 @@ int ertgb_lp_features(ertgb_ctx *ctx, float *x, float *f, void *stream) {
     return guard(c, [&] {
         if (!c->have_S) throw Error(ERTGB_STATE, "no assembled matrices (ertgb_assemble or a response first)");
         StreamJoin j(*c, stream);
-        lp_features(*c, x, f, c->stream);
+        with_less({c}, [&] { lp_features(*c, x, f, c->stream); });
         ERTGB_CUDA(cudaStreamSynchronize(c->stream));
         j.done();
     });
@@ -1021,52 +1133,8 @@ int ertgb_batch_response(ertgb_ctx *const *ctxs, int n, const double *const *rho
         }
         Context &c0 = *cs[0];
         ERTGB_CUDA(cudaSetDevice(c0.device));
-        for (Context *c : cs) {
-            if (c->rhs_align != 128) {
-                c->rhs_align = 128;
-                invalidate_derived(*c);
-            }
-            ensure_derived(*c);
-        }
-        // derived data (primary potentials, boundary terms, unit matrices) is
-        // built on each context's stream; the batch runs on the first one
-        for (Context *c : cs) ERTGB_CUDA(cudaStreamSynchronize(c->stream));
-        StreamJoin j(c0, stream);
-        cudaStream_t s = c0.stream;
-        ertgb_batch_info local{};
-        ertgb_batch_info *inf = info ? info : &local;
-        std::memset(inf, 0, sizeof(*inf));
-        ERTGB_CUDA(cudaEventRecord(c0.ev[0], s));
-        for (int i = 0; i < n; i++) {
-            Context &c = *cs[i];
-            c.have_pot = false;
-            c.stats = ertgb_stats{};
-            check_rho(c, rho[i], s);
-            c.d_rho_last = rho[i];
-            c.d_S.alloc((size_t)c.nK * c.mesh.nnz);
-            assemble_all(c, rho[i], c.d_S.p, s);
-            compute_source_rho(c, rho[i], s);
-            c.d_r.alloc((size_t)c.mesh.n * c.Rpad);
-            build_rhs(c, s);
-            compute_rhs_scale(c, s);
-            c.have_S = true;
-        }
-        ERTGB_CUDA(cudaEventRecord(c0.ev[1], s));
-        int stalled = 0;
-        const int status = batch_solve(cs, s, inf, &stalled);
-        inf->stalled_columns = stalled;
-        ERTGB_CUDA(cudaEventRecord(c0.ev[2], s));
-        for (int i = 0; i < n; i++) {
-            finish_potentials(*cs[i], s);
-            collect_response(*cs[i], rhoa[i], s);
-        }
-        ERTGB_CUDA(cudaEventRecord(c0.ev[3], s));
-        ERTGB_CUDA(cudaEventSynchronize(c0.ev[3]));
-        inf->ms_assemble = elapsed(c0, 0, 1);
-        inf->ms_solve = elapsed(c0, 1, 2);
-        inf->ms_collect = elapsed(c0, 2, 3);
-        for (Context *c : cs) c->have_pot = status == ERTGB_OK;
-        j.done();
+        int status = ERTGB_OK;
+        with_less(cs, [&] { status = batch_response(cs, rho, rhoa, info, stream); });
         if (status != ERTGB_OK) {
             set_free_error("batched solve did not converge within max_iter");
             return status;
@@ -1108,8 +1176,11 @@ int ertgb_response_complex(ertgb_ctx *ctx, const double *rho_re, const double *r
     return guard(c, [&] {
         ERTGB_REQUIRE(rho_re && rho_im && out_re && out_im, "null buffer");
         StreamJoin j(*c, stream);
-        ensure_derived(*c);
-        const int st = complex_response(*c, rho_re, rho_im, out_re, out_im, c->stream);
+        int st = ERTGB_OK;
+        with_less({c}, [&] {
+            ensure_derived(*c);
+            st = complex_response(*c, rho_re, rho_im, out_re, out_im, c->stream);
+        });
         j.done();
         if (st == ERTGB_NOT_CONVERGED) throw Error(ERTGB_NOT_CONVERGED, "complex COCG did not converge");
     });
@@ -1121,8 +1192,10 @@ int ertgb_jacobian_complex(ertgb_ctx *ctx, const double *m_re, const double *m_i
     return guard(c, [&] {
         ERTGB_REQUIRE(J, "null buffer");
         StreamJoin j(*c, stream);
-        ensure_derived(*c);
-        complex_jacobian(*c, m_re, m_im, n_model, J, c->stream);
+        with_less({c}, [&] {
+            ensure_derived(*c);
+            complex_jacobian(*c, m_re, m_im, n_model, J, c->stream);
+        });
         j.done();
     });
 }

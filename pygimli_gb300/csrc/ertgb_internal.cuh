@@ -35,6 +35,10 @@ struct Error : std::runtime_error {
         if (!(cond)) throw ::ertgb::Error(ERTGB_BAD_INPUT, msg);                           \
     } while (0)
 
+// Bytes held by the buffers that the calling thread allocated, and the most they
+// may come to (below 0: no limit; ertgb_alloc_limit).
+inline thread_local int64_t g_alloc_used = 0, g_alloc_limit = -1;
+
 // Owning device buffer (raw cudaMalloc; the library's own workspaces).
 template <class T> struct DBuf {
     T *p = nullptr;
@@ -45,6 +49,7 @@ template <class T> struct DBuf {
     ~DBuf() { release(); }
     void release() {
         if (p) cudaFree(p);
+        g_alloc_used -= (int64_t)(n * sizeof(T));
         p = nullptr;
         n = 0;
     }
@@ -52,8 +57,12 @@ template <class T> struct DBuf {
         if (count == n && p) return;
         release();
         if (count == 0) return;
+        const int64_t bytes = (int64_t)(count * sizeof(T));
+        if (g_alloc_limit >= 0 && g_alloc_used + bytes > g_alloc_limit)
+            throw Error(ERTGB_OOM, "the calling thread's limit on device memory");
         ERTGB_CUDA(cudaMalloc(&p, count * sizeof(T)));
         n = count;
+        g_alloc_used += bytes;
     }
     void upload(const T *h, size_t count, cudaStream_t s) {
         alloc(count);
@@ -321,6 +330,7 @@ struct Context {
     int precond = ERTGB_PRECOND_JACOBI;
     int precision = ERTGB_PRECISION_FP64;
     bool coarse_levels = true;    // multilevel preconditioner where it applies (ertgb_set_coarse_levels)
+    bool lean = false;            // without what only speed needs: the second try of a call that ran out of memory
     int rhs_align = 32;           // Rpad granularity (batches use 128)
     // derived per (mesh, electrodes, kw)
     int64_t R = 0, Rpad = 0;     // right-hand sides nK*nE, padded to 32
@@ -368,6 +378,10 @@ struct Context {
     ComplexState cx;
     ertgb_stats stats{};
 };
+
+// Releases what the context holds for speed only: coarse levels, the blocks of the
+// cyclic reduction, the solvers' z vectors.  The next solve allocates them again.
+void trim(Context &c);
 
 // --- launchers (defined in the .cu files) -----------------------------------
 // assemble.cu

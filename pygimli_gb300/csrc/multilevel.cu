@@ -418,9 +418,8 @@ void build(Context &c, cudaStream_t s) {
         for (int32_t v : c.calib) fixed[v] = 1;
     }
     if (M.tried && M.fixed == fixed) return;
-    M.tried = true;
+    M.tried = false;  // a failed allocation leaves it so: the next solve builds again
     M.ok = false;
-    M.fixed = fixed;
     M.levels.clear();
     // the unit-resistivity matrix
     std::vector<double> unit((size_t)m.nnz);
@@ -434,7 +433,11 @@ void build(Context &c, cudaStream_t s) {
     ERTGB_CUDA(cudaMemcpyAsync(unit.data(), src, sizeof(double) * unit.size(), cudaMemcpyDeviceToHost, s));
     ERTGB_CUDA(cudaStreamSynchronize(s));
     std::vector<HostLevel> H;
-    if (!build_levels(m.rowptr, m.colidx, unit, kMlCoarsest, kMlMaxLevels, H)) return;
+    if (!build_levels(m.rowptr, m.colidx, unit, kMlCoarsest, kMlMaxLevels, H)) {
+        M.tried = true;
+        M.fixed = fixed;
+        return;
+    }
     for (size_t k = 0; k < H.size(); k++) {
         auto l = std::make_unique<MlLevel>();
         const HostLevel &h = H[k];
@@ -468,7 +471,8 @@ void build(Context &c, cudaStream_t s) {
     M.bad.alloc(1);
     M.w.alloc(1);
     ERTGB_CUDA(cudaStreamSynchronize(s));  // host lists are freed on return
-    M.ok = true;
+    M.ok = M.tried = true;
+    M.fixed = fixed;
 }
 
 inline unsigned grid_rows(int64_t n, int per = kT) { return (unsigned)std::min<int64_t>(ceil_div(n, per), 1 << 16); }
@@ -562,22 +566,9 @@ template <typename T> static bool setup(Context &c, const double *fine, bool fac
 template <typename T>
 static bool guarded_setup(Context &c, const double *val, bool factor, int64_t cols, cudaStream_t s) {
     const MeshData &m = c.mesh;
-    if (!c.coarse_levels || m.dim != 3 || c.nK != 1 || c.k[0] != 0.0 || m.n < kMlMinRows) return false;
+    if (c.lean || !c.coarse_levels || m.dim != 3 || c.nK != 1 || c.k[0] != 0.0 || m.n < kMlMinRows) return false;
     if (!m.ext_rows.empty() || m.n_ext > 0) return false;
-    try {
-        return setup<T>(c, val, factor, cols, s);
-    } catch (Error &e) {
-        if (e.code != ERTGB_OOM) throw;
-        // the coarse levels do not fit beside the rest: the single-level form does without
-        cudaGetLastError();
-        Multilevel &M = c.mesh.ml;
-        M.levels.clear();
-        M.px.release();
-        M.pt.release();
-        M.pg.release();
-        M.ok = false;
-        return false;
-    }
+    return setup<T>(c, val, factor, cols, s);
 }
 
 bool ml_setup(Context &c, const double *val, bool factor, int64_t cols, cudaStream_t s) {

@@ -618,7 +618,7 @@ class ERTModelling:
             mr, mi = m[:len(m) // 2], m[len(m) // 2:]
         mr_d = torch.from_numpy(np.ascontiguousarray(mr)).to(dev)
         mi_d = torch.from_numpy(np.ascontiguousarray(mi)).to(dev)
-        J = torch.empty((self._data.size(), P), dtype=torch.complex128, device=dev)
+        J = self._empty_jacobian((self._data.size(), P), torch.complex128, dev)
         stream = torch.cuda.current_stream(dev).cuda_stream
         self._check(self._lib.ertgb_jacobian_complex(self._ctx, ctypes.c_void_p(mr_d.data_ptr()),
                                                      ctypes.c_void_p(mi_d.data_ptr()), int(len(mr)),
@@ -800,7 +800,7 @@ class ERTModelling:
             md = model.to(device=dev, dtype=torch.float64).contiguous()
         else:
             md = torch.from_numpy(np.ascontiguousarray(model, np.float64)).to(dev)
-        J = torch.empty((D, P), dtype=tdt, device=dev)
+        J = self._empty_jacobian((D, P), tdt, dev)
         stream = torch.cuda.current_stream(dev).cuda_stream
 
         def run():
@@ -815,6 +815,22 @@ class ERTModelling:
         self._check(rc)
         self._J = J
         return J
+
+    def _empty_jacobian(self, shape, dtype, dev):
+        """Device memory of a Jacobian; if it does not fit, once more without
+        what the operator keeps for speed only."""
+        torch = _torch()
+        try:
+            return torch.empty(shape, dtype=dtype, device=dev)
+        except torch.cuda.OutOfMemoryError:
+            self.trim()
+            return torch.empty(shape, dtype=dtype, device=dev)
+
+    def trim(self):
+        """Release the device memory that the operator keeps for speed only
+        (coarse levels, blocks of the banded solve); the next response takes it
+        again."""
+        self._check(self._lib.ertgb_trim(self._ctx))
 
     def _potentials_for_jacobian(self, model):
         """Sub-potentials for a Jacobian requested before any response
