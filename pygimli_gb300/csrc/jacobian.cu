@@ -971,11 +971,31 @@ static void build_stiff_plan(Context &c, int dt) {
     }
     // Node-wise table build (NS nodes per electrode) or the general one (a row per
     // node).  An odd NS spreads the staging's stores over the banks and may stage one
-    // node more than the tile has: with many electrodes that costs dipoles per chunk.
+    // node more than the tile has.  With 512 electrodes and more that leaves 5 % and
+    // more fewer dipoles per chunk, and the general build is taken where the node-wise
+    // one needs over 1.5 times its chunks: 756 electrodes (30 chunks against 15) 6.7
+    // and 5.0 ms, 841 (48 against 24) 7.4 and 5.5; 702 (17 against 12) 4.9 and 8.3,
+    // 624 (10 each) 3.9 and 4.3, 256 1.22 and 1.42
     const int NS = nl_tile | 1;
     const size_t rows = (size_t)nl_tile * row_bytes, nodes = ((size_t)(c.nE + 1) * NS * 8 + 15) / 16 * 16;
     auto cap_of = [&](size_t st) { return kStiffSmem < fixed + st ? (size_t)0 : (kStiffSmem - fixed - st) / per_dip; };
-    S.node_build = dt == 1 && NV <= 4 && nl_tile <= 32 && cap_of(nodes) >= 2 && 4 * cap_of(nodes) >= 3 * cap_of(rows);
+    auto chunks_of = [&](size_t cap) {  // of the data, as below
+        std::set<std::pair<int32_t, int32_t>> as, ms;
+        int64_t n = 1;
+        for (int64_t d = 0; d < c.D; d++) {
+            const int32_t *q = &c.abmn_h[4 * d];
+            as.insert({q[0], q[1]});
+            ms.insert({q[2], q[3]});
+            if (as.size() + ms.size() <= cap) continue;
+            n++;
+            as = {{q[0], q[1]}};
+            ms = {{q[2], q[3]}};
+        }
+        return n;
+    };
+    S.node_build = dt == 1 && NV <= 4 && nl_tile <= 32 && cap_of(nodes) >= 2;
+    if (S.node_build && c.nE >= 512 && cap_of(rows) >= 2)
+        S.node_build = 2 * chunks_of(cap_of(nodes)) <= 3 * chunks_of(cap_of(rows));
     const size_t stage = S.node_build ? nodes : rows;
     if (cap_of(stage) < 2) return;
     const size_t tab_cap = (kStiffSmem - fixed - stage) / 16 * 16;
