@@ -17,7 +17,6 @@
 #include <exception>
 #include <functional>
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 #include "ertgb_internal.cuh"
@@ -103,7 +102,7 @@ class Team {
         th_.reserve(kMost);
         try {
             for (int p = 1; p < want; p++) th_.emplace_back([this, p] { work(p); });
-        } catch (const std::system_error &) {  // no more threads: those that started do
+        } catch (const std::exception &) {  // no more threads or memory: those that started do
         }
     }
     ~Team() {
