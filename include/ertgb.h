@@ -223,7 +223,9 @@ int ertgb_analytic_potentials(ertgb_ctx *ctx, double rho);
  * as read by DataMap::data (core/src/bert/datamap.cpp:159-231). */
 int ertgb_set_scheme(ertgb_ctx *ctx, int n_data, const int32_t *abmn_host, const double *kfac_host);
 
-/* Solver controls: relative residual tolerance, iteration cap, preconditioner. */
+/* Solver controls: relative residual tolerance, iteration cap, preconditioner.
+ * With coarse levels (ertgb_set_coarse_levels) a solve goes on to a tenth of
+ * rtol, or to rtol where it no longer falls. */
 int ertgb_set_solver(ertgb_ctx *ctx, double rtol, int max_iter, int precond);
 /* Solver arithmetic (ertgb_precision).  No counterpart in the reference,
  * whose direct solver is FP64. */

@@ -207,8 +207,8 @@ __device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
 // k_jacobian holds the tables of all wavenumbers at once: on a 72-electrode line
 // (18 wavenumbers, 1330 distinct dipoles) one cell per block and five chunks
 // were left, bound by shared-memory conflicts and rebuilt tables.  Bound here:
-// the FP64 pipe, nv operations per distinct dipole and per pair for each
-// wavenumber and cell.  FP64 J: that line 44 -> 21.8 ms, 41
+// the FP64 pipe (75 % active on that line), nv operations per distinct dipole and
+// per pair for each wavenumber and cell.  FP64 J: that line 44 -> 21.8 ms, 41
 // electrodes (488 data, 76 dipoles) 0.74 -> 0.54; four cells per parameter (H2
 // forward mesh) 5.4 -> 2.0 ms, eight (3-D, 5336 data) 97 -> 20 ms.
 constexpr int kWT = 512;     // threads

@@ -4,7 +4,10 @@
 // of a 3-D potential problem to the CG recurrence: its iterations grow with
 // the mesh (FSAI 448 at 23k nodes, 1088 at 145k).  Coarse levels (coarsen.cpp)
 // take that error out; one symmetric V(1,1) cycle per iteration keeps the
-// count at 20-40.  Fine-level smoother: the chosen factor, w G^T G, or Jacobi;
+// count at 20-40 on log-normal ground of sigma 1, whatever the mesh.  P knows the
+// geometry only, so rough ground takes more (23k nodes, Jacobi / FSAI: 84 / 42 at
+// sigma 2, 126 / 60 at 3, 270 / 96 at 4; single level 1024 / 384, 2560 / 384 and
+// 4960 / 512).  Fine-level smoother: the chosen factor, w G^T G, or Jacobi;
 // Jacobi on the coarse levels; the dense inverse (FP64, at most 64 rows)
 // at the bottom.
 //
@@ -49,7 +52,7 @@ constexpr double kOmega = 1.5;        // damping against a spectrum bound of 1
 constexpr int kPower = 8;             // power iterations for the factor's damping
 constexpr float kPowerSafety = 1.1f;  // the Rayleigh quotient is a lower bound
 constexpr int kT = 256, kGroups = kT / 8;
-constexpr int64_t kFill = 304;        // blocks that fill the chip: two per SM
+constexpr int64_t kFill = 304;        // blocks that fill the chip: two on each of its 152 SMs
 
 // position of column c in the ascending row [q0, q1)
 __device__ __forceinline__ int32_t find_col(const int32_t *__restrict__ ci, int32_t q0, int32_t q1, int32_t c) {

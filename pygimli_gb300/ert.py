@@ -247,6 +247,9 @@ class ERTModelling:
         raise NotImplementedError("the linear solver is the built-in GPU block PCG")
 
     def setSolverTolerance(self, rtol=1e-10, maxIter=20000):
+        """Relative residual and iteration cap of the iterative solvers.  With
+        coarse levels (3-D, ``setCoarseLevels``) a solve goes on to a tenth of
+        ``rtol``, or to ``rtol`` where it no longer falls."""
         self._rtol, self._maxIter = float(rtol), int(maxIter)
         self._check(self._lib.ertgb_set_solver(self._ctx, self._rtol, self._maxIter, self._precond))
 
