@@ -241,9 +241,10 @@ int ertgb_set_coarse_levels(ertgb_ctx *ctx, int on);
  * allocation of its own that does not fit.  The next response takes the memory
  * again if it is free. */
 int ertgb_trim(ertgb_ctx *ctx);
-/* Limit, in bytes, on what the library buffers allocated by the calling thread
- * may hold (below 0: none, the default); beyond it a call meets ERTGB_OOM as if
- * the device were full.  used (may be null): what they hold now. */
+/* Bytes of device memory that the calling thread's library calls may take from
+ * now on, releases counted back (below 0: no limit, the default); beyond them a
+ * call meets ERTGB_OOM as if the device were full.  used (may be null): what the
+ * thread took less what it released so far. */
 int ertgb_alloc_limit(int64_t bytes, int64_t *used);
 
 /* Forward response: DCMultiElectrodeModelling::response

@@ -851,7 +851,7 @@ int ertgb_trim(ertgb_ctx *ctx) {
 }
 
 int ertgb_alloc_limit(int64_t bytes, int64_t *used) {
-    g_alloc_limit = bytes;
+    g_alloc_limit = bytes < 0 ? INT64_MAX : g_alloc_used + bytes;
     if (used) *used = g_alloc_used;
     return ERTGB_OK;
 }

@@ -35,9 +35,9 @@ struct Error : std::runtime_error {
         if (!(cond)) throw ::ertgb::Error(ERTGB_BAD_INPUT, msg);                           \
     } while (0)
 
-// Bytes held by the buffers that the calling thread allocated, and the most they
-// may come to (below 0: no limit; ertgb_alloc_limit).
-inline thread_local int64_t g_alloc_used = 0, g_alloc_limit = -1;
+// Bytes that the calling thread's buffers took less those that it released (below
+// 0 where another thread took them), and the most that may come to (ertgb_alloc_limit).
+inline thread_local int64_t g_alloc_used = 0, g_alloc_limit = INT64_MAX;
 
 // Owning device buffer (raw cudaMalloc; the library's own workspaces).
 template <class T> struct DBuf {
@@ -58,7 +58,7 @@ template <class T> struct DBuf {
         release();
         if (count == 0) return;
         const int64_t bytes = (int64_t)(count * sizeof(T));
-        if (g_alloc_limit >= 0 && g_alloc_used + bytes > g_alloc_limit)
+        if (g_alloc_used + bytes > g_alloc_limit)
             throw Error(ERTGB_OOM, "the calling thread's limit on device memory");
         ERTGB_CUDA(cudaMalloc(&p, count * sizeof(T)));
         n = count;

@@ -84,19 +84,18 @@ def test_response(torch, limit, form):
     del f
     gc.collect()
     f, rho = operator(form)
-    before = limit(-1)
-    limit(before + need - 1)  # the last allocation of the full form does not fit
+    before = limit(need - 1)  # the last allocation of the full form does not fit
     for _ in range(2):
         r = f.response(rho)
         v = potentials(f, r, cplx)
-        assert limit(before + need - 1) <= before + need - 1
+        assert limit(0) - before <= need - 1
+        limit(before + need - 1 - limit(0))
         assert float(np.max(np.abs(u - v).max(axis=-1) / np.abs(u).max(axis=-1))) <= 1e-8
         if "precond" not in form or form["precond"] != "band":
             assert f.stats()["iterations"] > 2 * st["iterations"]
     limit(-1)
     assert np.array_equal(f.response(rho), full) and f.stats()["iterations"] == st["iterations"]
-    limit(before + need // 4)  # what nothing can be done with stays an error
-    f.trim()
+    limit(need // 4)  # what nothing can be done with stays an error
     with pytest.raises(Exception, match="limit on device memory"):
         f2, _ = operator(form)
         f2.response(rho)
@@ -110,8 +109,7 @@ def test_jacobian(torch, limit, monkeypatch, form, dtype):
     J = f.createJacobian(rho, dtype=dtype)
     f, rho = operator(form)
     f.response(rho)
-    held = limit(-1)
-    limit(held)  # the library's scales (and split potentials) do not fit beside the solver's workspaces
+    held = limit(0)  # the library's scales (and split potentials) do not fit beside the solver's workspaces
     assert torch.equal(f.createJacobian(rho, dtype=dtype), J)
     assert limit(-1) < held
     f.response(rho)
@@ -134,8 +132,7 @@ def test_batch(torch, limit):
     fs, rhos = zip(*(operator(dict(precond="band")) for _ in range(2)))
     ref = [f.response(r) for f, r in zip(fs, rhos)]
     b = BatchedERTModelling(list(fs))
-    held = limit(-1)
-    limit(held)
+    limit(0)
     try:
         out = b.response(list(rhos))
     except Exception as e:  # even so it may not fit: the same error as ever, and the operators stay usable
