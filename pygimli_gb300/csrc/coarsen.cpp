@@ -326,7 +326,8 @@ bool build_levels(const std::vector<int32_t> &rowptr, const std::vector<int32_t>
                 if (a >= 0) a = a2[a];
             if (p + 1 < passes) W = collapse(team, W, a2, n2);
         }
-        if (n2 < 1 || n2 * 10 > U.n * 6) return false;  // the matching stalls: no useful hierarchy
+        // the matching stalls: no useful hierarchy (seen on H2 and P2 refinements, from 1667 rows downwards)
+        if (n2 < 1 || n2 * 10 > U.n * 6) return false;
         Csr P = prolongation(team, U, a1, n2), PT = transpose(P), AP = multiply(team, U, P);
         Csr C = multiply(team, PT, AP);
         HostLevel l;
