@@ -38,26 +38,34 @@ struct Csr {
 
 // one pass of pairwise matching in row order; returns the number of
 // aggregates.  A row without couplings (a fixed potential) joins none (-1): the
-// smoother alone solves it
-int64_t match(const Csr &A, double strong, std::vector<int32_t> &agg) {
+// smoother alone solves it.  join: a row whose partners are all taken goes to the
+// strongest one's aggregate instead of staying alone
+int64_t match(const Csr &A, double strong, bool join, std::vector<int32_t> &agg) {
     agg.assign((size_t)A.n, -1);
     int64_t na = 0;
     for (int64_t i = 0; i < A.n; i++) {
         if (agg[i] >= 0) continue;
         double strongest = 0.0, best = 0.0, off = 0.0;
-        int32_t with = -1;
+        int32_t with = -1, first = -1;
         for (int32_t q = A.rp[i]; q < A.rp[i + 1]; q++) {
             const int32_t j = A.ci[q];
             if (j == i) continue;
             const double c = -A.v[q];
             off += std::fabs(c);
-            strongest = std::max(strongest, c);
+            if (c > strongest) {
+                strongest = c;
+                first = j;
+            }
             if (agg[j] < 0 && c > best) {
                 best = c;
                 with = j;
             }
         }
         if (off == 0.0) continue;
+        if (join && with < 0 && first >= 0) {
+            agg[i] = agg[first];
+            continue;
+        }
         agg[i] = (int32_t)na;
         if (with >= 0 && best >= strong * strongest) agg[with] = (int32_t)na;
         na++;
@@ -315,19 +323,28 @@ bool build_levels(const std::vector<int32_t> &rowptr, const std::vector<int32_t>
     Team team(U.n);
     while (U.n > coarsest) {
         if ((int)out.size() >= max_levels) return false;
-        const double strong = U.n > kSmall ? kStrong : 0.0;
         const int passes = U.n > kTail ? 2 : 3;
         std::vector<int32_t> a1, a2;
-        int64_t n2 = match(U, strong, a1);
-        Csr W = collapse(team, U, a1, n2);
-        for (int p = 1; p < passes; p++) {
-            n2 = match(W, strong, a2);
-            for (auto &a : a1)
-                if (a >= 0) a = a2[a];
-            if (p + 1 < passes) W = collapse(team, W, a2, n2);
-        }
-        // the matching stalls: no useful hierarchy (seen on H2 and P2 refinements, from 1667 rows downwards)
-        if (n2 < 1 || n2 * 10 > U.n * 6) return false;
+        auto pair_up = [&](double strong, bool join) {
+            int64_t n2 = match(U, strong, join, a1);
+            Csr W = collapse(team, U, a1, n2);
+            for (int p = 1; p < passes; p++) {
+                n2 = match(W, strong, join, a2);
+                for (auto &a : a1)
+                    if (a >= 0) a = a2[a];
+                if (p + 1 < passes) W = collapse(team, W, a2, n2);
+            }
+            return n2;
+        };
+        int64_t n2 = pair_up(U.n > kSmall ? kStrong : 0.0, false);
+        auto stalls = [&] { return n2 < 1 || n2 * 10 > U.n * 6; };
+        // H2 and P2 refinements end in stars (rows that couple to one hub only, from
+        // some 1700 rows downwards), which pairs cannot collapse.  With the hierarchy given
+        // up there its construction was lost: first responses on the H2 mesh of a
+        // 16.6k-node box, 12 electrodes, FSAI, took 166 ms, 118 without coarse levels, 99
+        // so (P2: 273, 214, 128), repeated ones 115 and 43 (185 and 41).
+        if (stalls()) n2 = pair_up(0.0, true);
+        if (stalls()) return false;  // no useful hierarchy
         Csr P = prolongation(team, U, a1, n2), PT = transpose(P), AP = multiply(team, U, P);
         Csr C = multiply(team, PT, AP);
         HostLevel l;
